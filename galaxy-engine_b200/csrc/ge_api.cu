@@ -126,6 +126,7 @@ struct ge_ctx {
     std::vector<uint2> h_dtiles;
     std::vector<uint8_t> h_dflag;
     bool any_direct = false, any_walk = true;
+    int front = 0;                // front_plan of the current simulations
     uint32_t *d_err = nullptr;
     uint32_t *h_meta = nullptr;   // pinned copy of the tree meta words
     int64_t slots = 0;            // node slots of the last build (holes included)
@@ -624,6 +625,9 @@ int sync_segments(ge_ctx *c) {
     if (bb > (int64_t)c->num_sms * 4) bb = (int64_t)c->num_sms * 4;
     if (bb < 1) bb = 1;
     c->b.ss.box_blocks = (int)bb;
+    int64_t largest = 0;
+    for (const SimRec &s : c->sims) largest = std::max(largest, s.n);
+    c->front = front_plan(c->p.dims, largest, S);
     c->tree_valid = false;
     c->keys_valid = false;
     return direct_tables(c);
@@ -754,9 +758,27 @@ int enqueue_walk(ge_ctx *c, bool integrate_end) {
     return GE_OK;
 }
 
+// Everything before the build in one launch, where the simulations allow it.
+int enqueue_front(ge_ctx *c) {
+    GE_CHECK(c, launch_front(c->p.dims, c->front, cur_state(c), other_state(c), step_params(c),
+                             c->g, c->b.tree, c->b.ss, c->stream));
+    c->cur ^= 1;
+    return GE_OK;
+}
+
 int enqueue_frame(ge_ctx *c, cudaEvent_t *ev) {
     int rc;
     if (ev) GE_CHECK(c, cudaEventRecord(ev[0], c->stream));
+    if (c->front) {   // one stage: its time stands under the kick
+        if ((rc = enqueue_front(c))) return rc;
+        if (ev)
+            for (int k = 1; k <= 4; k++) GE_CHECK(c, cudaEventRecord(ev[k], c->stream));
+        if ((rc = enqueue_build(c, true))) return rc;
+        if (ev) GE_CHECK(c, cudaEventRecord(ev[5], c->stream));
+        if ((rc = enqueue_walk(c, true))) return rc;
+        if (ev) GE_CHECK(c, cudaEventRecord(ev[6], c->stream));
+        return GE_OK;
+    }
     if ((rc = enqueue_bbox(c, true))) return rc;
     if (ev) GE_CHECK(c, cudaEventRecord(ev[1], c->stream));
     if ((rc = enqueue_keys(c))) return rc;
@@ -916,9 +938,15 @@ int frame_overlapped(ge_ctx *c, int64_t n, const float *x, const float *y, const
         GE_CHECK(c, cudaEventRecord(c->xev[1], s1));
     }
     GE_CHECK(c, cudaEventRecord(c->ev[6], s0));
-    if ((rc = enqueue_bbox(c, true)) || (rc = enqueue_keys(c)) || (rc = enqueue_sort(c))) return rc;
-    GE_CHECK(c, cudaStreamWaitEvent(s0, c->xev[1], 0));
-    if ((rc = enqueue_permute(c, false))) return rc;
+    if (c->front) {
+        GE_CHECK(c, cudaStreamWaitEvent(s0, c->xev[1], 0));
+        if ((rc = enqueue_front(c))) return rc;
+    } else {
+        if ((rc = enqueue_bbox(c, true)) || (rc = enqueue_keys(c)) || (rc = enqueue_sort(c)))
+            return rc;
+        GE_CHECK(c, cudaStreamWaitEvent(s0, c->xev[1], 0));
+        if ((rc = enqueue_permute(c, false))) return rc;
+    }
     GE_CHECK(c, cudaEventRecord(c->xev[2], s0));
     GE_CHECK(c, cudaStreamWaitEvent(s1, c->xev[2], 0));
     {
@@ -1467,6 +1495,7 @@ std::vector<uint8_t> frame_signature(const ge_ctx *c) {
     put(&c->stream, sizeof c->stream);
     put(&c->d_err, sizeof c->d_err);
     put(&c->num_sms, sizeof c->num_sms);
+    put(&c->front, sizeof c->front);
     return v;
 }
 

@@ -12,68 +12,12 @@
 #include <cfloat>
 
 #include "ge_device.cuh"
+#include "ge_front_dev.cuh"
 #include "ge_internal.h"
 
 namespace ge {
 
 constexpr int kBoxBatch = 4;    // particles of a thread loaded together, before any store
-
-// float <-> unsigned with the same order (negative floats reversed)
-__device__ __forceinline__ uint32_t f2o(float f) {
-    const uint32_t u = __float_as_uint(f);
-    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ float o2f(uint32_t u) {
-    return __uint_as_float((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u);
-}
-
-// pos, vel, acc: particle i's, already loaded
-template <int D>
-__device__ __forceinline__ void kick_drift(const State &s, const StepParams &p, int i,
-                                           float *pos, float *vel, const float *acc) {
-    if (s.pvx) {
-        s.pvx[i] = vel[0]; s.pvy[i] = vel[1];
-        if (D == 3) s.pvz[i] = vel[2];
-    }
-    if (s.kx) {
-        // GE_PREC_MIXED: both updates Kahan-compensated
-        float *kp[3] = {s.kx, s.ky, s.kz}, *kv[3] = {s.kvx, s.kvy, s.kvz};
-#pragma unroll
-        for (int a = 0; a < D; a++) {
-            float cv = kv[a][i], cp = kp[a][i];
-            kahan_add(vel[a], cv, fmul(acc[a], p.half_dt));
-            kahan_add(pos[a], cp, fmul(vel[a], p.dt));
-            kv[a][i] = cv;
-            kp[a][i] = cp;
-        }
-    } else {
-#pragma unroll
-        for (int a = 0; a < D; a++) {
-            vel[a] = fadd(vel[a], fmul(acc[a], p.half_dt));   // vel += acc * halfDt
-            pos[a] = fadd(pos[a], fmul(vel[a], p.dt));         // pos += vel * dt
-        }
-    }
-    if (p.periodic) {
-        if (D == 2) {
-            // physics.cpp:1104-1110: domain [0, size)
-#pragma unroll
-            for (int a = 0; a < 2; a++) {
-                if (pos[a] < 0.0f) pos[a] = fadd(pos[a], p.domain[a]);
-                else if (pos[a] >= p.domain[a]) pos[a] = fsub(pos[a], p.domain[a]);
-            }
-        } else {
-            // physics3D.cpp:785-802: domain [-size/2, size/2)
-#pragma unroll
-            for (int a = 0; a < 3; a++) {
-                if (pos[a] < -p.half_domain[a]) pos[a] = fadd(pos[a], p.domain[a]);
-                else if (pos[a] >= p.half_domain[a]) pos[a] = fsub(pos[a], p.domain[a]);
-            }
-        }
-    }
-    s.x[i] = pos[0]; s.y[i] = pos[1];
-    s.vx[i] = vel[0]; s.vy[i] = vel[1];
-    if (D == 3) { s.z[i] = pos[2]; s.vz[i] = vel[2]; }
-}
 
 template <int D>
 __global__ void __launch_bounds__(kBBoxThreads)
@@ -190,14 +134,7 @@ __global__ void k_finalize_boxes(Segs g, Tree t, uint32_t n) {
         g.boxmm[sg * 6 + a] = 0xFFFFFFFFu;       // identity of min
         g.boxmm[sg * 6 + 3 + a] = 0u;            // identity of max
     }
-    float size = ref_max(fsub(h[0], l[0]), fsub(h[1], l[1]));
-    if (D == 3) size = ref_max(size, fsub(h[2], l[2]));
-    const float half = fmul(size, 0.5f);
-    float4 bb;
-    bb.x = fsub(fmul(fadd(l[0], h[0]), 0.5f), half);
-    bb.y = fsub(fmul(fadd(l[1], h[1]), 0.5f), half);
-    bb.z = D == 3 ? fsub(fmul(fadd(l[2], h[2]), 0.5f), half) : 0.0f;
-    bb.w = size;
+    const float4 bb = root_box<D>(l, h);
     g.box[sg] = bb;
     // root node of segment sg: cell = box, particle range = the segment
     t.cell[sg] = bb;

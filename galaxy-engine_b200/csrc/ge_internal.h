@@ -300,6 +300,14 @@ cudaError_t launch_sph_grid(const State &s, uint32_t lo, int n, float cell, uint
 // gather of the state into `out` by the sorted order
 cudaError_t launch_permute(int dims, int n, const SortScratch &ss, const State &in,
                            const State &out, bool with_acc, cudaStream_t st);
+// kick + drift, box, keys, sort and gather of every segment in one launch
+// (ge_front.cu), the state moving from `in` to `out`.  plan: what front_plan
+// chose for the largest segment's size and the number of segments (0: some
+// segment is too large for it, the passes run one by one).
+int front_plan(int dims, int64_t largest, int64_t sims);
+cudaError_t launch_front(int dims, int plan, const State &in, const State &out,
+                         const StepParams &p, const Segs &g, const Tree &t, SortScratch &ss,
+                         cudaStream_t st);
 // order (sorted slot -> previous index) copy-out for the stage API
 cudaError_t launch_perm_out(int dims, int n, const SortScratch &ss, uint32_t *perm,
                             cudaStream_t st);

@@ -21,6 +21,7 @@
 // status words (bounded waits).  Digit histograms of every pass are computed
 // once, by the key kernel.
 #include "ge_device.cuh"
+#include "ge_front_dev.cuh"
 #include "ge_internal.h"
 
 namespace ge {
@@ -35,20 +36,6 @@ constexpr uint32_t kFlagAgg = 1u << 30, kFlagInc = 2u << 30, kValMask = (1u << 3
 
 __host__ __device__ constexpr int key_passes(int dims) { return dims == 2 ? 4 : 7; }
 
-// The lanes whose BITS-bit digit equals this lane's, among the lanes with
-// `valid` set: one ballot per digit bit (the same mask as __match_any_sync
-// over the digits, for valid lanes; an invalid lane's mask is not used).
-template <int BITS>
-__device__ __forceinline__ unsigned digit_peers(uint32_t d, bool valid) {
-    unsigned m = __ballot_sync(0xffffffffu, valid);
-#pragma unroll
-    for (int b = 0; b < BITS; b++) {
-        const bool bit = (d >> b) & 1u;
-        const unsigned bb = __ballot_sync(0xffffffffu, bit);
-        m &= bit ? bb : ~bb;
-    }
-    return m;
-}
 static_assert(4 * kKeyBits == 36 && 7 * kKeyBits == 63, "passes cover the key bits");
 static_assert(7 * kKeyRadix <= kSortDigitWords, "hist / status words per segment / tile");
 static_assert(kKeyRadix <= kSortThreads, "one thread per digit");
@@ -101,28 +88,10 @@ k_keys(State s, int n, Segs g, uint64_t *keys, uint32_t *vals, uint32_t *hist,
         }
         uint64_t word = 0;
         if (ok) {
-            const float4 bb = g.box[sg];
-            float hx, hy, hz;
-            if (D == 2) {
-                const float ext = bb.w > 1e-6f ? bb.w : 1e-6f;   // std::max(posSize.z, 1e-6f)
-                hx = fadd(bb.x, ext); hy = fadd(bb.y, ext); hz = 0.0f;
-            } else {
-                hx = fadd(bb.x, bb.w); hy = fadd(bb.y, bb.w); hz = fadd(bb.z, bb.w);
-            }
-            if (D == 2) {
-                const uint64_t ix = scale_to_grid(s.x[i], bb.x, hx, 262144.0f, 262143ull);
-                const uint64_t iy = scale_to_grid(s.y[i], bb.y, hy, 262144.0f, 262143ull);
-                const uint64_t key = spread2(ix) | (spread2(iy) << 1);
-                word = (key << 28) | (uint64_t)i;
-                keys[i] = word;
-            } else {
-                const uint64_t ix = scale_to_grid(s.x[i], bb.x, hx, 2097151.0f, 2097151ull);
-                const uint64_t iy = scale_to_grid(s.y[i], bb.y, hy, 2097151.0f, 2097151ull);
-                const uint64_t iz = scale_to_grid(s.z[i], bb.z, hz, 2097151.0f, 2097151ull);
-                word = spread3(ix) | (spread3(iy) << 1) | (spread3(iz) << 2);
-                keys[i] = word;
-                vals[i] = (uint32_t)i;
-            }
+            word = morton_key<D>(g.box[sg], s.x[i], s.y[i], D == 3 ? s.z[i] : 0.0f);
+            if (D == 2) word = (word << 28) | (uint64_t)i;
+            else vals[i] = (uint32_t)i;
+            keys[i] = word;
         }
 #pragma unroll
         for (int ps = 0; ps < P; ps++) {
@@ -289,59 +258,17 @@ k_permute(const uint64_t *__restrict__ keys, const uint32_t *__restrict__ vals, 
     constexpr int U = kPermItems;
     const int stride = gridDim.x * blockDim.x * U;
     for (int k0 = blockIdx.x * blockDim.x * U + threadIdx.x; k0 < n; k0 += stride) {
-        int kk[U];
-        uint32_t j[U];
-        float x[U], y[U], z[U], vx[U], vy[U], vz[U], m[U], ax[U], ay[U], az[U];
-        uint32_t id[U];
+        uint32_t kk[U], j[U];
 #pragma unroll
         for (int u = 0; u < U; u++) {
-            kk[u] = k0 + u * (int)blockDim.x;
+            kk[u] = k0 + u * blockDim.x;
             j[u] = 0u;
-            if (kk[u] < n) {
+            if (kk[u] < (uint32_t)n) {
                 j[u] = (D == 2) ? (uint32_t)(keys[kk[u]] & 0x0FFFFFFFull) : vals[kk[u]];
-                if (j[u] >= (uint32_t)n) j[u] = (uint32_t)kk[u];   // only after a failed sort (error word set)
+                if (j[u] >= (uint32_t)n) j[u] = kk[u];   // only after a failed sort (error word set)
             }
         }
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            if (kk[u] >= n) continue;
-            const uint32_t q = j[u];
-            x[u] = in.x[q]; y[u] = in.y[q];
-            vx[u] = in.vx[q]; vy[u] = in.vy[q];
-            m[u] = in.m[q];
-            id[u] = in.id[q];
-            if (D == 3) { z[u] = in.z[q]; vz[u] = in.vz[q]; }
-            if (with_acc) {
-                ax[u] = in.ax[q]; ay[u] = in.ay[q];
-                if (D == 3) az[u] = in.az[q];
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            const int k = kk[u];
-            if (k >= n) continue;
-            const uint32_t q = j[u];
-            out.x[k] = x[u]; out.y[k] = y[u];
-            out.vx[k] = vx[u]; out.vy[k] = vy[u];
-            out.m[k] = m[u];
-            out.id[k] = id[u];
-            if (D == 3) { out.z[k] = z[u]; out.vz[k] = vz[u]; }
-            if (with_acc) {
-                out.ax[k] = ax[u]; out.ay[k] = ay[u];
-                if (D == 3) out.az[k] = az[u];
-            }
-            if (in.pvx) {
-                out.pvx[k] = in.pvx[q]; out.pvy[k] = in.pvy[q];
-                if (D == 3) out.pvz[k] = in.pvz[q];
-            }
-            if (in.pinned) out.pinned[k] = in.pinned[q];
-            if (in.temp) out.temp[k] = in.temp[q];
-            if (in.kx) {
-                out.kx[k] = in.kx[q]; out.ky[k] = in.ky[q];
-                out.kvx[k] = in.kvx[q]; out.kvy[k] = in.kvy[q];
-                if (D == 3) { out.kz[k] = in.kz[q]; out.kvz[k] = in.kvz[q]; }
-            }
-        }
+        gather_state<D, U, false>(in, out, with_acc, kk, j, (uint32_t)n);
     }
 }
 

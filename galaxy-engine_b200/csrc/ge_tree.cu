@@ -59,6 +59,14 @@ constexpr int kKmBlockQ = 33;   // key meta word: phase-1 nodes handed to the bl
 constexpr int kKmBlockTake = 34;   // key meta word: next block root to take
 constexpr int kKmProdDone = 64;    // key meta word (a cache line of its own): blocks done queueing
 
+// A pending count of one from the start: the node's other children (if any)
+// were final before anybody climbs, so its one pending child goes on without
+// the counter.  Set with the count, never counted down.
+constexpr uint32_t kSole = 0x80000000u;
+__device__ __forceinline__ uint32_t pend_word(uint32_t children) {
+    return children == 1u ? kSole | 1u : children;
+}
+
 // Bounded grid-wide barrier for a cooperative launch (all blocks resident).
 __device__ __forceinline__ void grid_barrier(uint32_t *bar_count, uint32_t *bar_gen,
                                              uint32_t *err) {
@@ -96,10 +104,21 @@ __device__ __forceinline__ void stamp(Tree &t) {
 
 
 // computeInternalMass / computeInternalMass3D: children read in the
-// reference's subGrids[x][y]([z]) order, x outermost
+// reference's subGrids[x][y]([z]) order, x outermost.  `own`: a child whose
+// entry is at hand in `mine` (kEmpty: none).
 template <int D>
-__device__ __forceinline__ float4 combine_children(const Tree &t, uint4 inf) {
+__device__ __forceinline__ float4 combine_children(const Tree &t, uint4 inf,
+                                                   uint32_t own = kEmpty,
+                                                   float4 mine = make_float4(0.f, 0.f, 0.f, 0.f)) {
     constexpr int Q = 1 << D;
+    // all children first (an absent one's load is the first child's again): a
+    // load inside the sum's branch is waited for there, one round trip each
+    float4 cw[Q];
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+        const bool has = (inf.y >> q) & 1u;
+        cw[q] = __ldcg(&t.walk[inf.x + (has ? __popc(inf.y & ((1u << q) - 1u)) : 0u)]);
+    }
     float gm = 0.0f, c[3] = {0.0f, 0.0f, 0.0f};
 #pragma unroll
     for (int kk = 0; kk < Q; kk++) {
@@ -107,13 +126,12 @@ __device__ __forceinline__ float4 combine_children(const Tree &t, uint4 inf) {
         if (D == 2) q = ((kk >> 1) & 1) | ((kk & 1) << 1);
         else q = ((kk >> 2) & 1) | (((kk >> 1) & 1) << 1) | ((kk & 1) << 2);
         if (!((inf.y >> q) & 1u)) continue;
-        const uint32_t ci = inf.x + __popc(inf.y & ((1u << q) - 1u));
-        const float4 cw = __ldcg(&t.walk[ci]);
-        const float cm = D == 2 ? cw.z : cw.w;
+        const float4 v = inf.x + __popc(inf.y & ((1u << q) - 1u)) == own ? mine : cw[q];
+        const float cm = D == 2 ? v.z : v.w;
         gm = fadd(gm, cm);
-        c[0] = fadd(c[0], fmul(cw.x, cm));
-        c[1] = fadd(c[1], fmul(cw.y, cm));
-        if (D == 3) c[2] = fadd(c[2], fmul(cw.z, cm));
+        c[0] = fadd(c[0], fmul(v.x, cm));
+        c[1] = fadd(c[1], fmul(v.y, cm));
+        if (D == 3) c[2] = fadd(c[2], fmul(v.z, cm));
     }
     if (gm > 0.0f) {
         c[0] = fdiv(c[0], gm); c[1] = fdiv(c[1], gm);
@@ -122,7 +140,7 @@ __device__ __forceinline__ float4 combine_children(const Tree &t, uint4 inf) {
     return make_float4(c[0], c[1], c[2], gm);
 }
 
-// Node k's mass is final: tell its parent.  The child that completes a
+// Node k's mass is final (kEmpty: nothing to do): tell its parent.  The child that completes a
 // parent's set combines the parent (in the reference's child order, so the
 // result does not depend on which child came last) and carries on upward.
 template <int D>
@@ -130,31 +148,43 @@ __device__ __forceinline__ void finish_upward(Tree &t, uint32_t k) {
     // the decrement releases this node's mass to the parent's last child,
     // whose decrement acquires every sibling's (one release sequence per counter).
     // An ancestor's links and cell were written before any of its children
-    // existed, so they are read ahead: the next ancestor's while this one's
-    // counter and children are on their way, which leaves two round trips
-    // (counter, children) per level.
+    // existed, so the next ancestor's are read ahead, before this one's
+    // counter, and leave two round trips (counter, children) per level; one
+    // (the children) where the node waited for this child alone (kSole), as
+    // most do: a node across one tile's edge, or in a chain.
+    if (k == kEmpty) return;
     uint32_t par = __ldcg(&t.aux[k]).z;
     if (par == kEmpty) return;
     uint4 inf = __ldcg(&t.info[par]);
     float size = __ldcg(&t.cell[par]).w;
     uint32_t next = __ldcg(&t.aux[par]).z;
+    uint32_t left = __ldcg(&t.pend[par]);
+    uint32_t own = kEmpty;
+    float4 mine = make_float4(0.f, 0.f, 0.f, 0.f);
     while (true) {
-        cuda::atomic_ref<uint32_t, cuda::thread_scope_device> pend(t.pend[par]);
-        if (pend.fetch_sub(1u, cuda::memory_order_acq_rel) != 1u) break;
         uint4 inf2 = make_uint4(0u, 0u, 0u, 0u);
         float size2 = 0.0f;
-        uint32_t next2 = kEmpty;
+        uint32_t next2 = kEmpty, left2 = 0u;
         if (next != kEmpty) {
             inf2 = __ldcg(&t.info[next]);
             size2 = __ldcg(&t.cell[next]).w;
             next2 = __ldcg(&t.aux[next]).z;
+            left2 = __ldcg(&t.pend[next]);
         }
-        put_walk<D>(t, par, combine_children<D>(t, inf), size);
+        if (!(left & kSole)) {
+            cuda::atomic_ref<uint32_t, cuda::thread_scope_device> pend(t.pend[par]);
+            if (pend.fetch_sub(1u, cuda::memory_order_acq_rel) != 1u) break;
+        }
+        const float4 cm = combine_children<D>(t, inf, own, mine);
+        put_walk<D>(t, par, cm, size);
         if (next == kEmpty) break;
+        own = par;
+        mine = D == 2 ? make_float4(cm.x, cm.y, cm.w, 0.0f) : cm;
         par = next;
         inf = inf2;
         size = size2;
         next = next2;
+        left = left2;
     }
 }
 
@@ -178,7 +208,7 @@ __device__ __forceinline__ void emit_children(Tree &t, uint32_t k, uint32_t firs
         ci++;
     }
     t.info[k] = make_uint4(first, mask, inf.z, inf.w);
-    atomicExch(&t.pend[k], (uint32_t)__popc(mask));
+    atomicExch(&t.pend[k], pend_word((uint32_t)__popc(mask)));
     __threadfence();
 }
 
@@ -279,7 +309,7 @@ __device__ __forceinline__ float4 write_chain(Tree &t, uint32_t first, uint32_t 
         atomicAdd(&t.endcnt[en], 1u);
         t.aux[k + 1] = make_uint4(cax.x + i + 1u, cax.y + i + 1u, k, 0u);
         t.info[k] = make_uint4(k + 1, 1u << q, st, en);
-        t.pend[k] = 1u;
+        t.pend[k] = pend_word(1u);
     }
     return cell;
 }
@@ -525,7 +555,7 @@ __device__ __forceinline__ void rebuild_level_node(const StepParams &p, Tree &t,
     }
     if (leader && ok) {
         t.info[k] = make_uint4(first, mask, inf.z, inf.w);
-        t.pend[k] = (uint32_t)__popc(mask);
+        t.pend[k] = pend_word((uint32_t)__popc(mask));
         if (j) {   // the chain's first node (write_chain writes and counts the rest)
             t.cell[first] = c1;
             t.aux[first] = make_uint4(ax.x + 1u, ax.y + 1u, k, 0u);
@@ -1040,7 +1070,7 @@ k_build(State s, StepParams p, Segs g, Tree t, uint32_t *err, int keyed) {
                 const uint32_t nch = (uint32_t)__popc(mask);
                 for (uint32_t c = 0; c < nch; c++) pending += (__ldcg(&t.aux[first + c]).w & 2u) ? 0u : 1u;
             }
-            t.pend[k] = pending;
+            t.pend[k] = pend_word(pending);
             const bool ready = !exact && !done && pending == 0u;
             // combined after the exact rebuilds: list them (slot_of is free
             // until the layout)
@@ -1122,6 +1152,7 @@ k_build(State s, StepParams p, Segs g, Tree t, uint32_t *err, int keyed) {
     }
     if ((*(volatile uint32_t *)err) & (kErrNodeCap | kErrSpin | kErrDepth)) return;
 
+    bool shared_roots = false;   // some block rebuilds a root
     if (keyed) {
         // exact-rebuild roots of up to kBlockRootMax particles: a block each
         // (shares its memory with phase 2's subtrees)
@@ -1129,6 +1160,7 @@ k_build(State s, StepParams p, Segs g, Tree t, uint32_t *err, int keyed) {
         // the nodes of 33 .. kBlockRootMax particles that phase 1 handed over
         // (its first level is the key passes' exact-rebuild roots)
         const uint32_t nblk = *(volatile uint32_t *)&t.kmeta[kKmBlockQ];
+        shared_roots = nblk > 0u;
         // slots come from phase 2's pool (above the phase-1 slots)
         const uint32_t xbase = le;
         uint32_t *xalloc = &t.meta[kMetaP2Alloc];
@@ -1137,13 +1169,10 @@ k_build(State s, StepParams p, Segs g, Tree t, uint32_t *err, int keyed) {
             sb.nout = 0u; sb.maxlev = 0u; sb.bad = 0u;
             sb.anext = sb.aend = sb.aused = 0u; sb.real = 0u; sb.hole_a = sb.hole_b = 0u;
         }
-        // roots taken one at a time from a counter (their costs differ)
-        while (true) {
-            __syncthreads();
-            if (threadIdx.x == 0) sb.r0 = atomicAdd(&t.kmeta[kKmBlockTake], 1u);
-            __syncthreads();
-            const uint32_t r = sb.r0;
-            if (r >= nblk) break;
+        // each block's first root by its number, the others one at a time from
+        // a counter (their costs differ)
+        uint32_t r = blockIdx.x;
+        while (r < nblk) {
             const uint32_t root = __ldcg(&t.kroots[nroots0 + r]);
             const uint4 ri = __ldcg(&t.info[root]);
             const uint32_t cnt = ri.w - ri.z;
@@ -1206,7 +1235,11 @@ k_build(State s, StepParams p, Segs g, Tree t, uint32_t *err, int keyed) {
                 cur ^= 1;
             }
             __syncthreads();
+            if (threadIdx.x == 0) sb.r0 = gridDim.x + atomicAdd(&t.kmeta[kKmBlockTake], 1u);
+            __syncthreads();
+            r = sb.r0;
         }
+        __syncthreads();
         if (threadIdx.x == 0) {
             flush_block_out<D>(t, sb, bid);
             if (sb.maxlev) atomicMax(&t.meta[kMetaLevels], sb.maxlev);
@@ -1250,17 +1283,20 @@ k_build(State s, StepParams p, Segs g, Tree t, uint32_t *err, int keyed) {
         return kNotYet;
     };
     // the listed key nodes whose children are all final (known since phase
-    // 0): combined and passed upward 32 at a time, by warps waiting for
-    // queue entries or done with them
+    // 0): combined and passed upward by warps waiting for queue entries or
+    // done with them
     const uint32_t nready = keyed ? *(volatile uint32_t *)&t.kmeta[5] : 0u;
     uint32_t *ready_ctr = &t.kmeta[kKeyMetaWords - 2];   // zeroed with the key passes' words
+    // (few per warp: the lanes of a warp wait for one another's round trips at
+    // every level)
+    const uint32_t rchunk = min(nready / nwarps + 1u, 32u);
     auto climb_ready = [&]() -> bool {   // false when none are left
         uint32_t b = 0;
-        if (lane == 0) b = atomicAdd(ready_ctr, 32u);
+        if (lane == 0) b = atomicAdd(ready_ctr, rchunk);
         b = __shfl_sync(0xffffffffu, b, 0);
         if (b >= nready) return false;
         const uint32_t idx = b + lane;
-        if (idx < nready) {
+        if (lane < rchunk && idx < nready) {
             const uint32_t cur = __ldcg(&t.slot_of[idx]);
             put_walk<D>(t, cur, combine_children<D>(t, __ldcg(&t.info[cur])),
                         __ldcg(&t.cell[cur]).w);
@@ -1276,8 +1312,12 @@ k_build(State s, StepParams p, Segs g, Tree t, uint32_t *err, int keyed) {
         // j-th finished subtree root whose upward pass is still to run, and the
         // warp runs 32 of them at once, so their atomics' round trips overlap
         uint32_t held = kEmpty, nheld = 0;
-        uint32_t task = 0;
-        if (lane == 0) task = atomicAdd(&t.meta[kMetaP2Task], 1u);
+        // without block roots every warp arrives at once, and its first task
+        // is its number's (a counter hands thousands of warps theirs one after
+        // another); with them the free warps take the tasks
+        const uint32_t task0 = shared_roots ? 0u : nwarps;
+        uint32_t task = gwarp;
+        if (shared_roots && lane == 0) task = atomicAdd(&t.meta[kMetaP2Task], 1u);
         bool ready_left = nready > 0;
         uint32_t ns = 32, spins = 0;
         while (true) {
@@ -1286,6 +1326,13 @@ k_build(State s, StepParams p, Segs g, Tree t, uint32_t *err, int keyed) {
             R = __shfl_sync(0xffffffffu, R, 0);
             if (R == kEmpty) break;
             if (R == kNotYet) {
+                if (nheld) {   // nothing to build meanwhile: upward with what is held
+                    finish_upward<D>(t, held);
+                    __syncwarp();
+                    held = kEmpty;
+                    nheld = 0;
+                    continue;
+                }
                 if (ready_left && (ready_left = climb_ready())) continue;
                 if (++spins > kSpinLimit) {
                     if (lane == 0) set_err(err, kErrSpin);
@@ -1296,7 +1343,7 @@ k_build(State s, StepParams p, Segs g, Tree t, uint32_t *err, int keyed) {
                 continue;
             }
             ns = 32;
-            if (lane == 0) task = atomicAdd(&t.meta[kMetaP2Task], 1u);
+            if (lane == 0) task = task0 + atomicAdd(&t.meta[kMetaP2Task], 1u);
             if (build_small_subtree_smem<D>(s, p, t, R, le, sm, wa, err)) {
                 if (lane == nheld) held = R;
                 if (++nheld == 32u) {
@@ -1311,7 +1358,7 @@ k_build(State s, StepParams p, Segs g, Tree t, uint32_t *err, int keyed) {
             __syncwarp();
         }
         __syncwarp();
-        if (held != kEmpty) finish_upward<D>(t, held);
+        finish_upward<D>(t, held);
         mark_holes(t, wa.next, wa.end);
         if (lane == 0 && wa.real) atomicAdd(&t.meta[kMetaReal], wa.real);
         while (ready_left && (ready_left = climb_ready())) {
@@ -1319,15 +1366,11 @@ k_build(State s, StepParams p, Segs g, Tree t, uint32_t *err, int keyed) {
     }
     if (keyed) {
         // the exact rebuilds' deferred leaves (already summed), upward from
-        // each, 32 at a time (the list is final once the queue is)
+        // each, few per warp (the list is final once the queue is)
         const uint32_t ndone = *(volatile uint32_t *)&t.kmeta[7];
-        uint32_t *take = &t.kmeta[kKeyMetaWords - 1];   // zeroed with the key passes' words
-        while (true) {
-            uint32_t b = 0;
-            if (lane == 0) b = atomicAdd(take, 32u);
-            b = __shfl_sync(0xffffffffu, b, 0);
-            if (b >= ndone) break;
-            if (b + lane < ndone) finish_upward<D>(t, __ldcg(&t.kdone[b + lane]));
+        const uint32_t dchunk = min(ndone / nwarps + 1u, 32u);
+        for (uint32_t b = gwarp * dchunk; b < ndone; b += nwarps * dchunk) {
+            if (lane < dchunk && b + lane < ndone) finish_upward<D>(t, __ldcg(&t.kdone[b + lane]));
             __syncwarp();
         }
     }
@@ -1496,8 +1539,12 @@ int build_grid_blocks(int dims, int num_sms) {
 cudaError_t launch_build(int dims, const State &s, const StepParams &p, const Segs &g, Tree &t,
                          uint32_t *err, int num_sms, cudaStream_t st, bool keyed) {
     // the kernel zeroes its own counters, level allocation and end histogram
-    const int blocks = build_grid_blocks(dims, num_sms);
+    // every block joins every barrier and polls: no more of them than one per
+    // 400 particles, and 64 (build stage of 2k particles 91 -> 74 us, 16k 102
+    // -> 89, 60k 161 -> 149 against the full grid)
+    int blocks = build_grid_blocks(dims, num_sms);
     if (blocks < 1) return cudaErrorLaunchOutOfResources;
+    blocks = min(blocks, max(64, (p.n + 399) / 400));
     State sc = s;
     StepParams pc = p;
     Segs gc = g;

@@ -106,7 +106,7 @@ template <int D>
 __global__ void __launch_bounds__(kMomThreads)
 k_moments(State s, Tree t, double inv_theta, uint32_t *err) {
     dep_wait();
-    constexpr int R = MomWords<D>::value;
+    constexpr int R = MomWords<D>::value, Q = 1 << D;
     const uint32_t slots = __ldcg(&t.meta[kMetaSlotsWord]);
     const uint32_t stride = gridDim.x * blockDim.x;
     const float *pos[3] = {s.x, s.y, s.z};
@@ -152,33 +152,53 @@ k_moments(State s, Tree t, double inv_theta, uint32_t *err) {
             if (pc.fetch_sub(1u, cuda::memory_order_acq_rel) != 1u) break;
             const uint4 pinf = __ldcg(&t.info[par]);
             const int nc = __popc(pinf.y);
+            const double *base = t.mom + (size_t)pinf.x * R;
+            // the children's masses and centres, then their moments, each in
+            // one go (an absent child's load is the first one's again): a load
+            // inside the sums is waited for there, a round trip per child
+            double mc[Q], cc[Q][D];
+#pragma unroll
+            for (int c = 0; c < Q; c++) {
+                const double *cr = base + (c < nc ? c * R : 0);
+                mc[c] = __ldcg(&cr[0]);
+#pragma unroll
+                for (int a = 0; a < D; a++) cc[c][a] = __ldcg(&cr[1 + a]);
+            }
             double q[R];
 #pragma unroll
             for (int w = 0; w < R; w++) q[w] = 0.0;
-            for (int c = 0; c < nc; c++) {
-                const double *cr = t.mom + (size_t)(pinf.x + (uint32_t)c) * R;
-                const double mc = __ldcg(&cr[0]);
-                q[0] += mc;
 #pragma unroll
-                for (int a = 0; a < D; a++) q[1 + a] = __fma_rn(mc, __ldcg(&cr[1 + a]), q[1 + a]);
+            for (int c = 0; c < Q; c++) {
+                if (c >= nc) continue;
+                q[0] += mc[c];
+#pragma unroll
+                for (int a = 0; a < D; a++) q[1 + a] = __fma_rn(mc[c], cc[c][a], q[1 + a]);
             }
             if (q[0] > 0.0) {
 #pragma unroll
                 for (int a = 0; a < D; a++) q[1 + a] /= q[0];
-                for (int c = 0; c < nc; c++) {
-                    const double *cr = t.mom + (size_t)(pinf.x + (uint32_t)c) * R;
-                    const double mc = __ldcg(&cr[0]);
-                    if (!(mc > 0.0)) continue;
-                    double d[3];
 #pragma unroll
-                    for (int a = 0; a < D; a++) d[a] = __ldcg(&cr[1 + a]) - q[1 + a];
+                for (int c0 = 0; c0 < Q; c0 += 4) {
+                    double mm[4][R - 1 - D];
 #pragma unroll
-                    for (int a = 0; a < D; a++)
+                    for (int c = 0; c < 4; c++)
 #pragma unroll
-                        for (int b = a; b < D; b++) {
-                            const int w = mom_index<D>(a, b);
-                            q[w] += __fma_rn(__dmul_rn(mc, d[a]), d[b], __ldcg(&cr[w]));
-                        }
+                        for (int w = 0; w < R - 1 - D; w++)
+                            mm[c][w] = __ldcg(&base[(c0 + c < nc ? (c0 + c) * R : 0) + 1 + D + w]);
+#pragma unroll
+                    for (int c = 0; c < 4; c++) {
+                        if (c0 + c >= nc || !(mc[c0 + c] > 0.0)) continue;
+                        double d[3];
+#pragma unroll
+                        for (int a = 0; a < D; a++) d[a] = cc[c0 + c][a] - q[1 + a];
+#pragma unroll
+                        for (int a = 0; a < D; a++)
+#pragma unroll
+                            for (int b = a; b < D; b++) {
+                                const int w = mom_index<D>(a, b);
+                                q[w] += __fma_rn(__dmul_rn(mc[c0 + c], d[a]), d[b], mm[c][w - 1 - D]);
+                            }
+                    }
                 }
             }
             double *prec = t.mom + (size_t)par * R;

@@ -21,17 +21,16 @@ namespace ge {
 constexpr int kTempThreads = 256;
 constexpr int kMetaSlotsT = 9;   // tree meta word: node slots of the last build
 
-__global__ void k_temp_pend_init(Tree t) {
+// the pending counts of every node, and the particles' own temperatures
+__global__ void __launch_bounds__(kTempThreads)
+k_temp_init(State s, Tree t, uint32_t n) {
+    dep_wait();
     const uint32_t slots = __ldcg(&t.meta[kMetaSlotsT]);
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < slots; k += stride) {
         const uint4 inf = __ldcg(&t.info[k]);
         t.pend[k] = (inf.w > inf.z) ? (uint32_t)__popc(inf.y) : 0u;
     }
-}
-
-__global__ void k_particle_temps(State s, Tree t, uint32_t n) {
-    const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += stride)
         t.tv[t.slot_of[j]] = s.temp[j];
 }
@@ -43,6 +42,7 @@ __device__ __forceinline__ void put_node_temp(const Tree &t, uint32_t k, float g
 
 template <int D>
 __global__ void __launch_bounds__(kTempThreads) k_node_temps(State s, Tree t) {
+    dep_wait();
     constexpr int Q = 1 << D;
     const uint32_t slots = __ldcg(&t.meta[kMetaSlotsT]);
     const uint32_t stride = gridDim.x * blockDim.x;
@@ -59,6 +59,14 @@ __global__ void __launch_bounds__(kTempThreads) k_node_temps(State s, Tree t) {
             cuda::atomic_ref<uint32_t, cuda::thread_scope_device> pc(t.pend[par]);
             if (pc.fetch_sub(1u, cuda::memory_order_acq_rel) != 1u) break;
             const uint4 pinf = __ldcg(&t.info[par]);
+            // all children's sums first (an absent one's load is the first's
+            // again): a load inside the sum is waited for there
+            float ct[Q];
+#pragma unroll
+            for (int q = 0; q < Q; q++) {
+                const bool has = (pinf.y >> q) & 1u;
+                ct[q] = __ldcg(&t.ntemp[pinf.x + (has ? __popc(pinf.y & ((1u << q) - 1u)) : 0u)]);
+            }
             float sum = 0.0f;
 #pragma unroll
             for (int kk = 0; kk < Q; kk++) {
@@ -67,7 +75,7 @@ __global__ void __launch_bounds__(kTempThreads) k_node_temps(State s, Tree t) {
                 if (D == 2) q = ((kk >> 1) & 1) | ((kk & 1) << 1);
                 else q = ((kk >> 2) & 1) | (((kk >> 1) & 1) << 1) | ((kk & 1) << 2);
                 if (!((pinf.y >> q) & 1u)) continue;
-                sum = fadd(sum, __ldcg(&t.ntemp[pinf.x + __popc(pinf.y & ((1u << q) - 1u))]));
+                sum = fadd(sum, ct[q]);
             }
             put_node_temp(t, par, sum, pinf.w - pinf.z);
             node = par;
@@ -78,14 +86,10 @@ __global__ void __launch_bounds__(kTempThreads) k_node_temps(State s, Tree t) {
 cudaError_t launch_node_temps(int dims, const State &s, const StepParams &p, Tree &t,
                               int num_sms, cudaStream_t st) {
     const int blocks = num_sms * 8;
-    k_temp_pend_init<<<blocks, kTempThreads, 0, st>>>(t);
-    cudaError_t e = cudaGetLastError();
+    const cudaError_t e = launch_dep(k_temp_init, blocks, kTempThreads, st, s, t, (uint32_t)p.n);
     if (e != cudaSuccess) return e;
-    k_particle_temps<<<blocks, kTempThreads, 0, st>>>(s, t, (uint32_t)p.n);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if (dims == 2) k_node_temps<2><<<blocks, kTempThreads, 0, st>>>(s, t);
-    else k_node_temps<3><<<blocks, kTempThreads, 0, st>>>(s, t);
-    return cudaGetLastError();
+    return dims == 2 ? launch_dep(k_node_temps<2>, blocks, kTempThreads, st, s, t)
+                     : launch_dep(k_node_temps<3>, blocks, kTempThreads, st, s, t);
 }
 
 }  // namespace ge

@@ -26,8 +26,7 @@ namespace {
 
 __device__ __forceinline__ float wrap_dd(float d, float dom, float hd) {
     // d -= domain * ((d > half) - (d < -half))   (physics.cpp:416-419)
-    const int k = (int)(d > hd) - (int)(d < -hd);
-    return fsub(d, fmul(dom, (float)k));
+    return fsub(d, d > hd ? dom : (d < -hd ? -dom : 0.0f));
 }
 
 __device__ __forceinline__ float rsqrt_fast(float x) {

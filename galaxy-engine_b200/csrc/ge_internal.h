@@ -68,6 +68,7 @@ struct State {
 //                   massless nodes: -2, both accepted by every opening test).  skip is where the walk
 //                   goes after accepting the entry: the successor of the node's
 //                   subtree, or the next entry for a particle.
+//                   (packed layout, below: 2D none, 3D uint32 entry words)
 //   slot_of uint32  entry index of each particle (for the self test)
 // The walk starts at entry 0 (the root) and ends at node_count + n.  The
 // positions need no top-down pass: with C(e) = #{nodes whose range ends at or
@@ -209,12 +210,14 @@ struct StepParams {
 // 2D walk entries {x, y, m, w}.  Plain layout: w = size^2 (-1 for a particle,
 // -2 for a massless node), the subtree successor in link[].  Packed layout
 // (tree meta word kMetaWalkPacked = 1): a node's w holds its level L (6 bits)
-// and its successor (26 bits); its size is the simulation's root size rs
-// halved L times (exact), so the plain layout's size^2 = fl(size_L^2) =
-// fl(rs^2) * 4^-L: fl(rs^2) with 2L taken off its exponent, exact while both
+// and how many entries past the next one its successor is (26 bits, so that a
+// walk moves forward whatever a word holds); its size is the simulation's root
+// size rs halved L times (exact), so the plain layout's size^2 = fl(size_L^2)
+// = fl(rs^2) * 4^-L: fl(rs^2) with 2L taken off its exponent, exact while both
 // are normal floats (every rs below 1e19 and min_size >= 1e-18, checked by
 // the build).  Massless nodes and particles carry the marker levels below
-// (L <= 46 for real levels); link[] holds every successor in both layouts.
+// (L <= 46 for real levels).  3D entries {x, y, z, m} have the same word in
+// link[], in place of the plain layout's {successor, size^2}.
 constexpr int kMetaWalkPacked = 13;
 // optional walk-layout arrays a build writes: each node's entry in aux.w (the
 // moment and node-temperature passes read it) and its entry range in nrange
@@ -229,8 +232,13 @@ __device__ __forceinline__ float packed_size2(uint32_t w_bits, uint32_t rs2_bits
     return __uint_as_float(rs2_bits - ((w_bits >> 2) & 0x3F000000u));   // exponent - 2L
 }
 constexpr uint32_t kPackSkipBits = 26, kPackMaxLevel = 46;
-__host__ __device__ constexpr uint32_t pack_entry_word(uint32_t level, uint32_t skip) {
-    return (level << kPackSkipBits) | skip;
+// entry k's word: `skip` is its successor
+__host__ __device__ constexpr uint32_t pack_entry_word(uint32_t level, uint32_t k, uint32_t skip) {
+    return (level << kPackSkipBits) | (skip - k - 1u);
+}
+// entries past the next one to its successor
+__host__ __device__ constexpr uint32_t packed_ahead(uint32_t w_bits) {
+    return w_bits & ((1u << kPackSkipBits) - 1u);
 }
 // Level values above kPackMaxLevel mark the packed entries that every opening
 // test accepts: a massless node (62; its successor follows) and a particle

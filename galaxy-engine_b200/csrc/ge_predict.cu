@@ -18,23 +18,24 @@ namespace ge {
 
 constexpr int kPredThreads = 64;
 
+// the packed layout's word of entry k: 2D in the entry, 3D in the link array
+__device__ __forceinline__ uint32_t entry_word(const Tree &t, int D, uint32_t k) {
+    return D == 2 ? __float_as_uint(__ldg(&t.src[k]).w) : __ldg(&((const uint32_t *)t.link)[k]);
+}
 // size^2 of entry k (-1 for a particle); rs_bits: the simulation's root
-// size^2, for the packed 2D layout
+// size^2, for the packed layout
 __device__ __forceinline__ float entry_s2(const Tree &t, int D, uint32_t k, bool packed,
                                           uint32_t rs_bits) {
-    if (D == 3) return __uint_as_float(__ldg(&((const uint2 *)t.link)[k]).y);
-    const float4 A = __ldg(&t.src[k]);
-    if (!packed) return A.w;
-    const uint32_t wb = __float_as_uint(A.w);
+    if (!packed)
+        return D == 2 ? __ldg(&t.src[k]).w : __uint_as_float(__ldg(&((const uint2 *)t.link)[k]).y);
+    const uint32_t wb = entry_word(t, D, k);
     if (packed_particle(wb)) return -1.0f;
     if (packed_accepts(wb)) return -2.0f;   // a massless node
     return packed_size2(wb, rs_bits);
 }
-// successor of entry k (A = its src word): packed 2D entries carry it in
-// their fourth word's low bits (no link array is written then)
-__device__ __forceinline__ uint32_t entry_skip(const Tree &t, int D, uint32_t k, bool packed,
-                                               float4 A) {
-    if (D == 2 && packed) return __float_as_uint(A.w) & ((1u << kPackSkipBits) - 1u);
+// successor of entry k
+__device__ __forceinline__ uint32_t entry_skip(const Tree &t, int D, uint32_t k, bool packed) {
+    if (packed) return k + 1u + packed_ahead(entry_word(t, D, k));
     return D == 2 ? __ldg(&((const uint32_t *)t.link)[k]) : __ldg(&((const uint2 *)t.link)[k]).x;
 }
 
@@ -46,7 +47,7 @@ __device__ void old_force(const Tree &t, const StepParams &p, uint32_t begin, ui
     uint32_t k = begin;
     while (k < end) {
         const float4 A = __ldg(&t.src[k]);
-        const uint32_t skip = entry_skip(t, D, k, packed, A);
+        const uint32_t skip = entry_skip(t, D, k, packed);
         const uint32_t nxt = max(k + 1, skip);   // always moves forward
         const float gm = D == 2 ? A.z : A.w;
         if (!(gm > 0.0f)) { k = nxt; continue; }   // gridMass <= 0: skip the subtree
@@ -94,7 +95,7 @@ k_predict(Tree t, StepParams p, const float4 *box, uint32_t begin, uint32_t end,
           const float *__restrict__ mass, int steps, float *__restrict__ path) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= nprobes) return;
-    const bool packed = D == 2 && __ldg(&t.meta[kMetaWalkPacked]) != 0u;
+    const bool packed = __ldg(&t.meta[kMetaWalkPacked]) != 0u;
     const float rs = packed ? __ldg(box).w : 0.0f;   // the simulation's root size
     const uint32_t rs_bits = __float_as_uint(fmul(rs, rs));
     float ps[3] = {0.f, 0.f, 0.f}, v[3] = {0.f, 0.f, 0.f}, F[3];

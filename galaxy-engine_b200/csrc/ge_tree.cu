@@ -969,16 +969,17 @@ __device__ __forceinline__ void scatter_entry(const State &s, const Segs &g, Tre
         // it is accepted by every test (size^2 = -2; particles have -1),
         // carries no mass (the walk makes no interaction with a massless
         // node) and leads to its successor.
-        t.src[me] = D == 2 ? make_float4(w.x, w.y, 0.0f,
-                                         packed ? __uint_as_float(pack_entry_word(kPackMassless, skip))
-                                                : -2.0f)
+        const uint32_t word = packed ? pack_entry_word(kPackMassless, me, skip) : 0u;
+        t.src[me] = D == 2 ? make_float4(w.x, w.y, 0.0f, packed ? __uint_as_float(word) : -2.0f)
                            : make_float4(w.x, w.y, w.z, 0.0f);
-        if (D == 3) ((uint2 *)t.link)[me] = make_uint2(skip, __float_as_uint(-2.0f));
+        if (D == 3 && packed) ((uint32_t *)t.link)[me] = word;
+        else if (D == 3) ((uint2 *)t.link)[me] = make_uint2(skip, __float_as_uint(-2.0f));
         else if (!packed) ((uint32_t *)t.link)[me] = skip;
     } else {
-        t.src[me] = D == 2 && packed ? make_float4(w.x, w.y, w.z, __uint_as_float(pack_entry_word(ax.x, skip)))
-                                     : w;
-        if (D == 3) ((uint2 *)t.link)[me] = make_uint2(skip, __float_as_uint(size2));
+        const uint32_t word = packed ? pack_entry_word(ax.x, me, skip) : 0u;
+        t.src[me] = D == 2 && packed ? make_float4(w.x, w.y, w.z, __uint_as_float(word)) : w;
+        if (D == 3 && packed) ((uint32_t *)t.link)[me] = word;
+        else if (D == 3) ((uint2 *)t.link)[me] = make_uint2(skip, __float_as_uint(size2));
         else if (!packed) ((uint32_t *)t.link)[me] = skip;
     }
     if (inf.y) return;
@@ -1003,12 +1004,13 @@ __device__ __forceinline__ void scatter_entry(const State &s, const Segs &g, Tre
             if (massless) continue;   // never reached by the walk
             if (D == 2) {
                 t.src[e] = make_float4(px[q], py[q], pm[q],
-                                       packed ? __uint_as_float(pack_entry_word(kPackParticle, e + 1))
+                                       packed ? __uint_as_float(pack_entry_word(kPackParticle, e, e + 1))
                                               : -1.0f);
                 if (!packed) ((uint32_t *)t.link)[e] = e + 1;
             } else {
                 t.src[e] = make_float4(px[q], py[q], pz[q], pm[q]);
-                ((uint2 *)t.link)[e] = make_uint2(e + 1, __float_as_uint(-1.0f));
+                if (packed) ((uint32_t *)t.link)[e] = pack_entry_word(kPackParticle, e, e + 1);
+                else ((uint2 *)t.link)[e] = make_uint2(e + 1, __float_as_uint(-1.0f));
             }
         }
     }
@@ -1460,12 +1462,12 @@ k_build(State s, StepParams p, Segs g, Tree t, uint32_t *err, int keyed) {
     //   subtree successor    = C(end) + level - same_end + end
     //   entry of particle j  = entry of its leaf + 1 + (j - start)
     const uint32_t total = nodes + n;
-    // 2D, not rewritten by the moment pass: packed entries when every level
+    // unless the moment pass rewrites them: packed entries when every level
     // and successor fits the word and every size^2 is a normal float (a node
     // of size <= min_size is a leaf, so sizes stay >= min_size / 2, or the
     // tree is one leaf; root sizes below 1e19), where quartering L times is
     // the exponent minus 2L
-    const bool packed = D == 2 && !p.mixed && p.min_size >= 1e-18f &&
+    const bool packed = !p.mixed && p.min_size >= 1e-18f &&
                         *(volatile uint32_t *)&t.meta[kMetaBigRoot] == 0u &&
                         *(volatile uint32_t *)&t.meta[kMetaLevels] <= kPackMaxLevel + 1u &&
                         total < (1u << kPackSkipBits);

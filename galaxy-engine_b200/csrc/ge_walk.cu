@@ -38,15 +38,18 @@
 
 namespace ge {
 
-// threads per block: 1024 in 3D, where a block's particles (consecutive in
-// Morton order, on one SM) share more of their longer walks through L1
-// (3.70 -> 3.42 ms for the 1M Plummer walk against 256); 256 in 2D (no gain)
-template <int D> constexpr int walk_threads() { return D == 2 ? 256 : 1024; }
+// Threads per block: a block's particles, consecutive in Morton order on one
+// SM, share most of their walks through L1, so small systems take no smaller
+// blocks (16k in 2D: 51 us, 59 with 64 threads).  (1024 in 3D shared more while
+// a link had 8 bytes, 1M 1.65 ms against 1.78; with packed links 256 takes
+// 1.56, 250k 483 us against 537, 60k 188 against 275, 16k 142 against 227.)
+constexpr int kWalkThreads = 256;
 
 __device__ __forceinline__ float wrap_d(float d, float dom, float hd) {
-    // d -= domain * ((d > half) - (d < -half))   (physics.cpp:118-121)
-    const int k = (int)(d > hd) - (int)(d < -hd);
-    return fsub(d, fmul(dom, (float)k));
+    // d -= domain * ((d > half) - (d < -half))   (physics.cpp:118-121), the
+    // factor -1, 0 or 1 by selection: its conversion to float would go through
+    // the unit that the reciprocal square root needs
+    return fsub(d, d > hd ? dom : (d < -hd ? -dom : 0.0f));
 }
 
 __device__ __forceinline__ float rsqrt_approx(float x) {
@@ -66,8 +69,38 @@ template <int D> struct LinkOf;
 template <> struct LinkOf<2> { using T = uint32_t; };
 template <> struct LinkOf<3> { using T = uint2; };
 
+// The 2D packed walk of entries [k, end) in FAST arithmetic, not periodic,
+// eps2 > 0: the terms of massless sources and of the particle itself add
+// exactly zero.  x and y go through packed operations (f32x2), each rounded as
+// the scalar one.  The loads' L1 wavefronts bound it (79 % of peak; 6.7 per
+// load, the lanes of a warp at some five entries), so a quarter fewer
+// instructions give little: 1M at theta 0.7 278 -> 276 us, 283 in the general
+// loop.
+__device__ __forceinline__ void walk_packed2(const float4 *__restrict__ src, uint32_t k,
+                                             uint32_t end, uint32_t rs2_bits, const float *pi,
+                                             float eps2, float th2, float *f) {
+    const f32x2 np = pack2(-pi[0], -pi[1]);
+    f32x2 fxy = pack2(0.0f, 0.0f);
+    while (k < end) {
+        const ulonglong2 A = __ldg(reinterpret_cast<const ulonglong2 *>(src + k));
+        float m, w;
+        unpack2(A.y, m, w);
+        const uint32_t wb = __float_as_uint(w);
+        const f32x2 d = add2(A.x, np);
+        float xx, yy;
+        unpack2(mul2(d, d), xx, yy);
+        const float r2 = fadd(fadd(xx, yy), eps2);
+        const bool acc = (int)(rs2_bits - ((wb >> 2) & 0x3F000000u)) < __float_as_int(fmul(th2, r2));
+        const float inv = rsqrt_approx(r2);
+        const float fm = acc ? m * (inv * inv * inv) : 0.0f;
+        fxy = fma2(d, pack2(fm, fm), fxy);
+        k += 1u + (acc ? packed_ahead(wb) : 0u);
+    }
+    unpack2(fxy, f[0], f[1]);
+}
+
 template <int D, int MODE, bool COUNT, bool PER, bool POS_EPS, bool TEMP = false>
-__global__ void __launch_bounds__(walk_threads<D>())
+__global__ void __launch_bounds__(kWalkThreads)
 k_walk(State s, StepParams p, Segs g, Tree t, int integrate_end, unsigned long long *inter,
        uint32_t *err) {
     dep_wait();
@@ -96,27 +129,29 @@ k_walk(State s, StepParams p, Segs g, Tree t, int integrate_end, unsigned long l
         uint32_t k = __ldg(&g.root_begin[sg]);
         const uint32_t end = __ldg(&g.root_end[sg]);
         uint32_t cnt = 0;
-        // 2D packed entries: one load per step (the successor and the level
-        // in the fourth word); the root size of the particle's simulation
-        const bool packed = D == 2 && MODE != GE_PREC_MIXED && __ldg(&t.meta[kMetaWalkPacked]) != 0u;
+        // packed entries: the successor and the level in one word; the root
+        // size of the particle's simulation
+        const bool packed = MODE != GE_PREC_MIXED && __ldg(&t.meta[kMetaWalkPacked]) != 0u;
         const float rs = packed ? __ldg(&g.box[sg]).w : 0.0f;
         const uint32_t rs2_bits = __float_as_uint(fmul(rs, rs));   // the root's size^2
         // the loop once per layout, chosen here rather than at every step
         auto walk_range = [&](auto pk) {
-            constexpr bool PK = decltype(pk)::value && D == 2 && MODE != GE_PREC_MIXED;
+            constexpr bool PK = decltype(pk)::value && MODE != GE_PREC_MIXED;
             while (k < end) {
                 const float4 A = __ldg(&src[k]);
                 const float m = D == 2 ? A.z : A.w;
                 float s2;          // a node's size^2 (plain layout: -1 particle, -2 massless)
-                uint32_t nxt_skip;
+                uint32_t nxt_skip = 0u;
+                uint32_t ahead = 0u;   // packed: entries past the next one to the successor
                 bool part;         // a particle's entry
                 bool always = false;   // packed: a particle or a massless node
                 if constexpr (PK) {
-                    const uint32_t wb = __float_as_uint(A.w);
+                    const uint32_t wb = D == 2 ? __float_as_uint(A.w)
+                                               : __ldg(&((const uint32_t *)t.link)[k]);
                     always = packed_accepts(wb);
                     part = packed_particle(wb);
                     s2 = packed_size2(wb, rs2_bits);   // not used for marked entries
-                    nxt_skip = wb & ((1u << kPackSkipBits) - 1u);   // a particle's: k + 1
+                    ahead = packed_ahead(wb);          // a particle's: none
                 } else {
                     const LT L = __ldg(&link[k]);
                     s2 = link_s2(L, A.w);
@@ -227,11 +262,21 @@ k_walk(State s, StepParams p, Segs g, Tree t, int integrate_end, unsigned long l
                 }
                 // a valid skip lies past k; max() keeps k increasing whatever the
                 // layout holds, so the walk ends within end - begin entries (a
-                // packed particle's own successor is k + 1)
-                if constexpr (PK) k = max(k + 1, acc ? nxt_skip : k + 1);
+                // packed word cannot point back)
+                if constexpr (PK) k = k + 1u + (acc ? ahead : 0u);
                 else k = max(k + 1, acc && !part ? nxt_skip : k + 1);
             }
         };
+        if constexpr (!kSelfTest && D == 2 && !PER) {
+            // As signed words the size^2 of a node and theta^2 r2 compare as
+            // the floats do, and a marker level (62 or 63 off the root's
+            // exponent) lies below theta^2 r2 whenever it lies below theta^2
+            // eps2: one subtraction and one compare decide every entry.
+            if (packed && (int)(rs2_bits - (kPackMassless << 24)) < __float_as_int(fmul(th2, eps2))) {
+                walk_packed2(src, k, end, rs2_bits, pi, eps2, th2, f);
+                k = end;
+            }
+        }
         if (packed) walk_range(std::true_type{});
         else walk_range(std::false_type{});
         float a3[3];
@@ -264,7 +309,6 @@ k_walk(State s, StepParams p, Segs g, Tree t, int integrate_end, unsigned long l
 template <int D, int MODE, bool COUNT, bool PER, bool POS_EPS, bool TEMP = false>
 static cudaError_t walk_one(const State &s, const StepParams &p, const Segs &g, const Tree &t,
                             int ie, unsigned long long *inter, uint32_t *err, cudaStream_t st) {
-    constexpr int kWalkThreads = walk_threads<D>();
     const int blocks = (p.n - p.i0 + kWalkThreads - 1) / kWalkThreads;
     return launch_dep(k_walk<D, MODE, COUNT, PER, POS_EPS, TEMP>, blocks < 1 ? 1 : blocks,
                       kWalkThreads, st, s, p, g, t, ie, inter, err);

@@ -67,6 +67,23 @@ k_aos_out(unsigned char *__restrict__ phys, AosLayout L, int n, State s,
     }
 }
 
+// Whole arrays into page-locked host memory, stored over PCIe by the kernel:
+// one launch where copies would be queued one by one (each some 4 us of the
+// copy engine's own latency).
+__global__ void __launch_bounds__(256) k_store_arrays(HostArrays h, int n) {
+    const uint32_t *src = h.src[blockIdx.y];
+    uint32_t *dst = h.dst[blockIdx.y];
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        dst[i] = src[i];
+}
+
+cudaError_t launch_store_arrays(const HostArrays &h, int n, cudaStream_t st) {
+    int b = (n + 255) / 256;
+    if (b > 32) b = 32;
+    k_store_arrays<<<dim3(b, h.count), 256, 0, st>>>(h, n);
+    return cudaGetLastError();
+}
+
 static int aos_grid(int n) {
     int b = (n + 255) / 256;
     if (b > 148 * 16) b = 148 * 16;

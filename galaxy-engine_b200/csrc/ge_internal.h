@@ -268,6 +268,15 @@ cudaError_t launch_aos_in(int dims, const unsigned char *phys, const unsigned ch
 cudaError_t launch_aos_out(int dims, unsigned char *phys, const AosLayout &L, int n,
                            const State &s, const SortScratch &ss, cudaStream_t st);
 
+// n words of each device array src[q] to dst[q], page-locked host memory as the
+// device addresses it
+struct HostArrays {
+    int count;
+    const uint32_t *src[11];
+    uint32_t *dst[11];
+};
+cudaError_t launch_store_arrays(const HostArrays &h, int n, cudaStream_t st);
+
 // --- launchers (each runs on `st`) ----------------------------------------
 // integrateStart (kick + drift) fused with the per-segment bounding-box
 // reduction; a second small kernel applies the reference's box formula per

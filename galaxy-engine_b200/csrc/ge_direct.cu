@@ -13,9 +13,15 @@
 //   GE_PREC_EXACT : the scalar form's rounding (correctly rounded sqrt and
 //                   division, no contraction): bit-identical to it.
 //   GE_PREC_FAST  : approximate reciprocal square root and FMA accumulation.
-// A block takes kDirectTile particles of one simulation and streams that
+// EXACT: a block takes kDirectTile particles of one simulation and streams that
 // simulation's particles through shared memory in order, so every thread
 // accumulates in the reference's j order.
+// FAST: the simulations this pass is for have some thousand particles, so one
+// thread per particle leaves most SMs idle and each thread a serial sum of
+// thousands of terms.  A block takes 32 particles, its 8 warps an eighth of
+// the sources each (every 8th run of 32), and the 8 partial sums are added in
+// warp order: 8 times the threads, sums an eighth as long, the same result
+// alone and in a batch.
 #include "ge_bh.h"
 #include "ge_device.cuh"
 #include "ge_internal.h"
@@ -35,9 +41,10 @@ __device__ __forceinline__ float rsqrt_fast(float x) {
     return r;
 }
 
-template <int D, int MODE, bool PER>
+template <int D, bool PER>
 __global__ void __launch_bounds__(kDirectTile)
 k_direct(State s, StepParams p, Segs g, const uint2 *__restrict__ tiles, int integrate_end) {
+    dep_wait();
     __shared__ float4 sj[kDirectTile];   // {x, y, z, G * m}
     const uint2 tile = tiles[blockIdx.x];
     const uint32_t lo = seg_lo(g, tile.x), hi = seg_hi(g, tile.x, (uint32_t)p.n);
@@ -68,17 +75,10 @@ k_direct(State s, StepParams p, Segs g, const uint2 *__restrict__ tiles, int int
                 float r2 = fadd(fmul(d[0], d[0]), fmul(d[1], d[1]));
                 if (D == 3) r2 = fadd(r2, fmul(d[2], d[2]));
                 r2 = fadd(r2, soft);
-                if (MODE == GE_PREC_EXACT) {
-                    const float inv = fdiv(1.0f, __fsqrt_rn(r2));
-                    const float f = fmul(q.w, fmul(fmul(inv, inv), inv));
+                const float inv = fdiv(1.0f, __fsqrt_rn(r2));
+                const float f = fmul(q.w, fmul(fmul(inv, inv), inv));
 #pragma unroll
-                    for (int a = 0; a < D; a++) acc[a] = fadd(acc[a], fmul(d[a], f));
-                } else {
-                    const float inv = rsqrt_fast(r2);
-                    const float f = q.w * (inv * inv * inv);
-#pragma unroll
-                    for (int a = 0; a < D; a++) acc[a] = fmaf(d[a], f, acc[a]);
-                }
+                for (int a = 0; a < D; a++) acc[a] = fadd(acc[a], fmul(d[a], f));
             }
         }
         __syncthreads();
@@ -93,14 +93,97 @@ k_direct(State s, StepParams p, Segs g, const uint2 *__restrict__ tiles, int int
     }
 }
 
-template <int D, int MODE>
-cudaError_t direct_mode(const State &s, const StepParams &p, const Segs &g, const uint2 *tiles,
-                        int64_t ntiles, int ie, cudaStream_t st) {
-    if (p.periodic)
-        k_direct<D, MODE, true><<<(unsigned)ntiles, kDirectTile, 0, st>>>(s, p, g, tiles, ie);
-    else
-        k_direct<D, MODE, false><<<(unsigned)ntiles, kDirectTile, 0, st>>>(s, p, g, tiles, ie);
-    return cudaGetLastError();
+constexpr int kDfWarps = 8, kDfThreads = 32 * kDfWarps;
+constexpr int kDfSub = kDirectTile / 32;   // blocks per tile of the table
+constexpr int kDfStage = 2 * kDfThreads;   // sources staged at a time
+
+template <int D, bool PER>
+__global__ void __launch_bounds__(kDfThreads)
+k_direct_fast(State s, StepParams p, Segs g, const uint2 *__restrict__ tiles, int integrate_end) {
+    dep_wait();
+    __shared__ float4 sj[kDfStage];   // {x, y, z, G * m}
+    __shared__ float part[kDfWarps][3][32];
+    const uint2 tile = tiles[blockIdx.x / kDfSub];
+    const uint32_t lo = seg_lo(g, tile.x), hi = seg_hi(g, tile.x, (uint32_t)p.n);
+    const uint32_t first = tile.y + (blockIdx.x % kDfSub) * 32u;
+    if (first >= hi) return;   // the whole block
+    const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31u, i = first + lane;
+    const bool own = i < hi;
+    float pi[3] = {0.f, 0.f, 0.f};
+    if (own) {
+        pi[0] = s.x[i]; pi[1] = s.y[i];
+        if (D == 3) pi[2] = s.z[i];
+    }
+    const float soft = p.direct_eps2;
+    float acc[3] = {0.f, 0.f, 0.f};
+    float4 next[2];   // the next stage's sources, on their way during this one's sums
+    auto load = [&](uint32_t base) {
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const uint32_t j = base + u * kDfThreads + threadIdx.x;
+            next[u] = j < hi ? make_float4(s.x[j], s.y[j], D == 3 ? s.z[j] : 0.0f, fmul(p.G, s.m[j]))
+                             : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+    load(lo);
+    for (uint32_t base = lo; base < hi; base += kDfStage) {
+        __syncthreads();
+        sj[threadIdx.x] = next[0];
+        sj[kDfThreads + threadIdx.x] = next[1];
+        __syncthreads();
+        load(base + kDfStage);
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const uint32_t t0 = u * kDfThreads + w * 32u;
+            if (base + t0 >= hi) break;
+            const int cnt = (int)min(32u, hi - (base + t0));
+#pragma unroll 8
+            for (int t = 0; t < cnt; t++) {
+                const float4 q = sj[t0 + t];
+                float d[3] = {fsub(q.x, pi[0]), fsub(q.y, pi[1]), D == 3 ? fsub(q.z, pi[2]) : 0.f};
+                if (PER) {
+#pragma unroll
+                    for (int a = 0; a < D; a++) d[a] = wrap_dd(d[a], p.domain[a], p.half_domain[a]);
+                }
+                float r2 = fadd(fmul(d[0], d[0]), fmul(d[1], d[1]));
+                if (D == 3) r2 = fadd(r2, fmul(d[2], d[2]));
+                r2 = fadd(r2, soft);
+                const float inv = rsqrt_fast(r2);
+                const float f = q.w * (inv * inv * inv);
+#pragma unroll
+                for (int a = 0; a < D; a++) acc[a] = fmaf(d[a], f, acc[a]);
+            }
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < D; a++) part[w][a][lane] = acc[a];
+    __syncthreads();
+    if (w != 0 || !own) return;
+#pragma unroll
+    for (int a = 0; a < D; a++) {
+        acc[a] = part[0][a][lane];
+#pragma unroll
+        for (int q = 1; q < kDfWarps; q++) acc[a] += part[q][a][lane];
+    }
+    s.ax[i] = acc[0]; s.ay[i] = acc[1];
+    if (D == 3) s.az[i] = acc[2];
+    if (integrate_end && !(s.pinned && s.pinned[i])) {
+        s.vx[i] = fadd(s.vx[i], fmul(acc[0], p.half_dt));
+        s.vy[i] = fadd(s.vy[i], fmul(acc[1], p.half_dt));
+        if (D == 3) s.vz[i] = fadd(s.vz[i], fmul(acc[2], p.half_dt));
+    }
+}
+
+template <int D>
+cudaError_t direct_dims(bool exact, const State &s, const StepParams &p, const Segs &g,
+                        const uint2 *tiles, int64_t ntiles, int ie, cudaStream_t st) {
+    if (!exact) {
+        const unsigned blocks = (unsigned)(ntiles * kDfSub);
+        return p.periodic ? launch_dep(k_direct_fast<D, true>, blocks, kDfThreads, st, s, p, g, tiles, ie)
+                          : launch_dep(k_direct_fast<D, false>, blocks, kDfThreads, st, s, p, g, tiles, ie);
+    }
+    return p.periodic ? launch_dep(k_direct<D, true>, (unsigned)ntiles, kDirectTile, st, s, p, g, tiles, ie)
+                      : launch_dep(k_direct<D, false>, (unsigned)ntiles, kDirectTile, st, s, p, g, tiles, ie);
 }
 
 }  // namespace
@@ -111,11 +194,8 @@ cudaError_t launch_direct(int dims, int precision, const State &s, const StepPar
     if (ntiles <= 0) return cudaSuccess;
     const int ie = integrate_end ? 1 : 0;
     const bool exact = precision == GE_PREC_EXACT;
-    if (dims == 2)
-        return exact ? direct_mode<2, GE_PREC_EXACT>(s, p, g, tiles, ntiles, ie, st)
-                     : direct_mode<2, GE_PREC_FAST>(s, p, g, tiles, ntiles, ie, st);
-    return exact ? direct_mode<3, GE_PREC_EXACT>(s, p, g, tiles, ntiles, ie, st)
-                 : direct_mode<3, GE_PREC_FAST>(s, p, g, tiles, ntiles, ie, st);
+    return dims == 2 ? direct_dims<2>(exact, s, p, g, tiles, ntiles, ie, st)
+                     : direct_dims<3>(exact, s, p, g, tiles, ntiles, ie, st);
 }
 
 }  // namespace ge

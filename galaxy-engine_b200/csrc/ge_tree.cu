@@ -964,6 +964,7 @@ __device__ __forceinline__ void scatter_entry(const State &s, const Segs &g, Tre
     }
     const float nm = D == 2 ? w.z : w.w;
     const bool massless = nm <= 0.0f;
+    bool negative = nm < 0.0f;
     if (massless) {
         // gridMass <= 0: the reference skips the whole subtree.  As a source
         // it is accepted by every test (size^2 = -2; particles have -1),
@@ -982,7 +983,10 @@ __device__ __forceinline__ void scatter_entry(const State &s, const Segs &g, Tre
         else if (D == 3) ((uint2 *)t.link)[me] = make_uint2(skip, __float_as_uint(size2));
         else if (!packed) ((uint32_t *)t.link)[me] = skip;
     }
-    if (inf.y) return;
+    if (inf.y) {
+        if (negative) t.meta[kMetaNegMass] = 1u;
+        return;
+    }
     // a leaf: its particles follow it, four at a time (loads before stores)
     for (uint32_t j0 = inf.z; j0 < inf.w; j0 += 4u) {
         float px[4], py[4], pz[4], pm[4];
@@ -994,6 +998,7 @@ __device__ __forceinline__ void scatter_entry(const State &s, const Segs &g, Tre
             py[q] = in ? s.y[j] : 0.0f;
             pz[q] = in && D == 3 ? s.z[j] : 0.0f;
             pm[q] = in ? s.m[j] : 0.0f;
+            negative = negative || pm[q] < 0.0f;
         }
 #pragma unroll
         for (int q = 0; q < 4; q++) {
@@ -1014,6 +1019,7 @@ __device__ __forceinline__ void scatter_entry(const State &s, const Segs &g, Tre
             }
         }
     }
+    if (negative) t.meta[kMetaNegMass] = 1u;
 }
 
 template <int D>
@@ -1048,7 +1054,7 @@ k_build(State s, StepParams p, Segs g, Tree t, uint32_t *err, int keyed) {
         t.meta[kMetaNodes] = 0u; t.meta[kMetaLevels] = 0u;
         t.meta[kMetaSmall] = 0u; t.meta[kMetaP2Alloc] = 0u; t.meta[kMetaTimeline] = 0u;
         t.meta[kMetaReal] = 0u; t.meta[kMetaSlots] = 0u; t.meta[kMetaP2Task] = 0u;
-        t.meta[kMetaBigRoot] = 0u; t.meta[kMetaDone] = 0u; t.kmeta[kKmProdDone] = 0u;
+        t.meta[kMetaBigRoot] = 0u; t.meta[kMetaNegMass] = 0u; t.meta[kMetaDone] = 0u; t.kmeta[kKmProdDone] = 0u;
         const uint32_t id = t.meta[kMetaBuildId] + 1u;   // read after the first grid barrier
         t.meta[kMetaBuildId] = id ? id : 1u;
         stamp(t);

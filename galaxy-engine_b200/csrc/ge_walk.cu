@@ -52,6 +52,27 @@ __device__ __forceinline__ float wrap_d(float d, float dom, float hd) {
     return fsub(d, d > hd ? dom : (d < -hd ? -dom : 0.0f));
 }
 
+// Whether no offset from a particle to anything inside its simulation's root
+// box can pass half the domain, so that the wrap leaves every offset as it is.
+// Centres of mass lie in the box when no mass is negative, up to their sums'
+// rounding: the margin (5 % of half the domain, coordinates up to twice the
+// domain) covers plain sums of 10^5 coincident particles.  In a 3D sphere of
+// 250k reaching 77 % of the domain this holds for most particles: walk 566 ->
+// 477 us; a 2D disk of 1M well inside it 421 -> 271 (no wrap at all: 271).
+template <int D>
+__device__ __forceinline__ bool never_wraps(const Tree &t, const float4 &box, const StepParams &p,
+                                            const float *x) {
+    const float lo[3] = {box.x, box.y, box.z};
+    bool in = __ldg(&t.meta[kMetaNegMass]) == 0u;
+#pragma unroll
+    for (int a = 0; a < D; a++) {
+        const float most = 0.95f * p.half_domain[a];
+        in = in && x[a] - lo[a] < most && lo[a] + box.w - x[a] < most &&
+             fabsf(lo[a]) + box.w < 4.0f * p.half_domain[a];
+    }
+    return in;
+}
+
 __device__ __forceinline__ float rsqrt_approx(float x) {
     float r;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -135,7 +156,8 @@ k_walk(State s, StepParams p, Segs g, Tree t, int integrate_end, unsigned long l
         const float rs = packed ? __ldg(&g.box[sg]).w : 0.0f;
         const uint32_t rs2_bits = __float_as_uint(fmul(rs, rs));   // the root's size^2
         // the loop once per layout, chosen here rather than at every step
-        auto walk_range = [&](auto pk) {
+        auto walk_range = [&](auto pk, auto wrap) {
+            constexpr bool WRAP = decltype(wrap)::value;
             constexpr bool PK = decltype(pk)::value && MODE != GE_PREC_MIXED;
             while (k < end) {
                 const float4 A = __ldg(&src[k]);
@@ -162,7 +184,7 @@ k_walk(State s, StepParams p, Segs g, Tree t, int integrate_end, unsigned long l
                 d[0] = fsub(A.x, pi[0]);
                 d[1] = fsub(A.y, pi[1]);
                 d[2] = D == 3 ? fsub(A.z, pi[2]) : 0.0f;
-                if (PER) {
+                if (WRAP) {
     #pragma unroll
                     for (int a = 0; a < D; a++) d[a] = wrap_d(d[a], p.domain[a], p.half_domain[a]);
                 }
@@ -267,18 +289,29 @@ k_walk(State s, StepParams p, Segs g, Tree t, int integrate_end, unsigned long l
                 else k = max(k + 1, acc && !part ? nxt_skip : k + 1);
             }
         };
-        if constexpr (!kSelfTest && D == 2 && !PER) {
+        // a periodic walk whose offsets cannot wrap is the plain one
+        const bool wraps = PER && !never_wraps<D>(t, g.box[sg], p, pi);
+        if constexpr (!kSelfTest && D == 2) {
             // As signed words the size^2 of a node and theta^2 r2 compare as
             // the floats do, and a marker level (62 or 63 off the root's
             // exponent) lies below theta^2 r2 whenever it lies below theta^2
             // eps2: one subtraction and one compare decide every entry.
-            if (packed && (int)(rs2_bits - (kPackMassless << 24)) < __float_as_int(fmul(th2, eps2))) {
+            if (!wraps && packed &&
+                (int)(rs2_bits - (kPackMassless << 24)) < __float_as_int(fmul(th2, eps2))) {
                 walk_packed2(src, k, end, rs2_bits, pi, eps2, th2, f);
                 k = end;
             }
         }
-        if (packed) walk_range(std::true_type{});
-        else walk_range(std::false_type{});
+        auto by_layout = [&](auto wrap) {
+            if (packed) walk_range(std::true_type{}, wrap);
+            else walk_range(std::false_type{}, wrap);
+        };
+        if constexpr (PER) {
+            if (wraps) by_layout(std::true_type{});
+            else by_layout(std::false_type{});
+        } else {
+            by_layout(std::false_type{});
+        }
         float a3[3];
 #pragma unroll
         for (int a = 0; a < D; a++)
@@ -306,9 +339,170 @@ k_walk(State s, StepParams p, Segs g, Tree t, int integrate_end, unsigned long l
     }
 }
 
+// ---- 3D FAST: two particles per thread --------------------------------------
+// Two Morton neighbours visit nearly the same entries (4 % more together than
+// either alone), so a thread that walks for both loads each entry once: the
+// loads' L1 wavefronts are what bounds the 3D walk.  The thread stands at entry
+// k for both; a particle that accepts an entry which the other opens takes the
+// monopole and sits out the subtree (until entry ra / rb).  Each particle meets
+// exactly its own entries, in its own order, with the single walk's arithmetic:
+// the same bits.  Half the threads and a longer step, so it pays where the walks
+// are long and many: walk (us), single / pairs, theta 0.7: 60k 190 / 227, 150k
+// 268 / 283, 200k 383 / 332, 250k 479 / 397, 1M 1558 / 1334; theta 0.5 1M 5172 /
+// 3588; theta 1.0 150k 119 / 150, 400k 283 / 275; periodic (a warp that holds
+// both kinds of particles runs both loops) 250k 477 / 520, 1M 1580 / 1438.  In
+// 2D, bound by instructions as much as by L1, it does not (1M 277 / 285).
+constexpr int kPairThreads = 128;
+static bool walk_pairs(const StepParams &p) {
+    const int n = p.n - p.i0;
+    return n >= 400000 || (n >= 200000 && p.theta <= 0.8f && !p.periodic);
+}
+
+// entry k in either layout: whether a particle at squared distance r2
+// (softened) accepts it, and its successor
+__device__ __forceinline__ bool entry_accepts3(const Tree &t, uint32_t k, bool packed,
+                                               uint32_t rs2_bits, float th2r2, uint32_t &nxt) {
+    if (packed) {
+        const uint32_t wb = __ldg(&((const uint32_t *)t.link)[k]);
+        nxt = k + 1u + packed_ahead(wb);
+        return packed_accepts(wb) || packed_size2(wb, rs2_bits) < th2r2;
+    }
+    const uint2 l = __ldg(&((const uint2 *)t.link)[k]);
+    nxt = max(k + 1u, l.x);   // a particle's successor is k + 1
+    return __uint_as_float(l.y) < th2r2;
+}
+
+template <bool PER>
+__global__ void __launch_bounds__(kPairThreads)
+k_walk_pair(State s, StepParams p, Segs g, Tree t, int integrate_end) {
+    dep_wait();
+    const float eps2 = p.eps2, th2 = p.theta2, G = p.G;
+    const uint32_t n = (uint32_t)p.n;
+    const uint32_t i0 = (uint32_t)p.i0 + 2u * (blockIdx.x * blockDim.x + threadIdx.x);
+    if (i0 >= n) return;
+    const bool packed = __ldg(&t.meta[kMetaWalkPacked]) != 0u;
+    const float4 *__restrict__ src = t.src;
+    const uint32_t *__restrict__ link = (const uint32_t *)t.link;
+    const uint32_t i[2] = {i0, min(i0 + 1u, n - 1u)};
+    uint32_t sg[2];
+    bool on[2];   // a particle of the launch that takes the walk
+    f32x2 np[2], f[2] = {pack2(0.f, 0.f), pack2(0.f, 0.f)};
+    float pz[2], fz[2] = {0.f, 0.f};
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        sg[q] = g.seg_of ? __ldg(&g.seg_of[i[q]]) : 0u;
+        on[q] = i0 + q < n && !(g.direct && __ldg(&g.direct[sg[q]]));
+        np[q] = pack2(-s.x[i[q]], -s.y[i[q]]);
+        pz[q] = s.z[i[q]];
+    }
+    // both together inside one simulation, else one after the other
+    const bool one = sg[0] == sg[1];
+#pragma unroll 1
+    for (int pass = one ? 2 : 0; pass < (one ? 3 : 2); pass++) {
+        // the entry each particle is waiting for (kEmpty: not walking now)
+        uint32_t r[2] = {on[0] && pass != 1 ? 0u : kEmpty, on[1] && pass != 0 ? 0u : kEmpty};
+        if (r[0] & r[1]) continue;   // neither
+        const uint32_t sgp = pass == 1 ? sg[1] : sg[0];
+        uint32_t k = __ldg(&g.root_begin[sgp]);
+        const uint32_t end = __ldg(&g.root_end[sgp]);
+        const float rs = __ldg(&g.box[sgp]).w;
+        const uint32_t rs2_bits = __float_as_uint(fmul(rs, rs));
+        // (the signed compare that decides packed entries, marker levels too, as
+        // in the 2D packed walk; otherwise the entry's own test)
+        const bool by_word =
+            packed && (int)(rs2_bits - (kPackMassless << 24)) < __float_as_int(fmul(th2, eps2));
+        auto walk = [&](auto words, auto wrap) {
+          constexpr bool WORDS = decltype(words)::value, WRAP = decltype(wrap)::value;
+          while (k < end) {
+            const ulonglong2 A = __ldg(reinterpret_cast<const ulonglong2 *>(src + k));
+            float z, m;
+            unpack2(A.y, z, m);
+            f32x2 d[2];
+            float dz[2], r2[2];
+            bool acc[2];
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                d[q] = add2(A.x, np[q]);
+                dz[q] = fsub(z, pz[q]);
+                if (WRAP) {
+                    float dx, dy;
+                    unpack2(d[q], dx, dy);
+                    d[q] = pack2(wrap_d(dx, p.domain[0], p.half_domain[0]),
+                                 wrap_d(dy, p.domain[1], p.half_domain[1]));
+                    dz[q] = wrap_d(dz[q], p.domain[2], p.half_domain[2]);
+                }
+                float xx, yy;
+                unpack2(mul2(d[q], d[q]), xx, yy);
+                r2[q] = fadd(fadd(fadd(xx, yy), fmul(dz[q], dz[q])), eps2);
+            }
+            uint32_t nxt;
+            if constexpr (WORDS) {
+                const uint32_t wb = __ldg(link + k);
+                const int s2 = (int)(rs2_bits - ((wb >> 2) & 0x3F000000u));
+                nxt = k + 1u + packed_ahead(wb);
+#pragma unroll
+                for (int q = 0; q < 2; q++) acc[q] = s2 < __float_as_int(fmul(th2, r2[q]));
+            } else {
+#pragma unroll
+                for (int q = 0; q < 2; q++)
+                    acc[q] = entry_accepts3(t, k, packed, rs2_bits, fmul(th2, r2[q]), nxt);
+            }
+            bool open = false;
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                const bool here = k >= r[q], take = acc[q] && here;
+                const float inv = rsqrt_approx(r2[q]);
+                const float fm = take ? m * (inv * inv * inv) : 0.0f;
+                f[q] = fma2(d[q], pack2(fm, fm), f[q]);
+                fz[q] = fmaf(dz[q], fm, fz[q]);
+                r[q] = take ? nxt : r[q];
+                open |= here && !acc[q];
+            }
+            k = open ? k + 1u : nxt;
+          }
+        };
+        auto by_layout = [&](auto wrap) {
+            if (by_word) walk(std::true_type{}, wrap);
+            else walk(std::false_type{}, wrap);
+        };
+        bool wraps = false;
+        if (PER)
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                const float x[3] = {s.x[i[q]], s.y[i[q]], pz[q]};
+                wraps = wraps || !never_wraps<3>(t, g.box[sgp], p, x);
+            }
+        if constexpr (PER) {
+            if (wraps) by_layout(std::true_type{});
+            else by_layout(std::false_type{});
+        } else {
+            by_layout(std::false_type{});
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        if (!on[q]) continue;
+        float a3[3];
+        unpack2(f[q], a3[0], a3[1]);
+        a3[0] = G * a3[0];
+        a3[1] = G * a3[1];
+        a3[2] = G * fz[q];
+        s.ax[i[q]] = a3[0]; s.ay[i[q]] = a3[1]; s.az[i[q]] = a3[2];
+        if (integrate_end && !(s.pinned && s.pinned[i[q]])) {
+            s.vx[i[q]] = fadd(s.vx[i[q]], fmul(a3[0], p.half_dt));
+            s.vy[i[q]] = fadd(s.vy[i[q]], fmul(a3[1], p.half_dt));
+            s.vz[i[q]] = fadd(s.vz[i[q]], fmul(a3[2], p.half_dt));
+        }
+    }
+}
+
 template <int D, int MODE, bool COUNT, bool PER, bool POS_EPS, bool TEMP = false>
 static cudaError_t walk_one(const State &s, const StepParams &p, const Segs &g, const Tree &t,
                             int ie, unsigned long long *inter, uint32_t *err, cudaStream_t st) {
+    if constexpr (D == 3 && MODE == GE_PREC_FAST && !COUNT && POS_EPS && !TEMP)
+        if (walk_pairs(p))
+            return launch_dep(k_walk_pair<PER>, (p.n - p.i0 + 2 * kPairThreads - 1) / (2 * kPairThreads),
+                              kPairThreads, st, s, p, g, t, ie);
     const int blocks = (p.n - p.i0 + kWalkThreads - 1) / kWalkThreads;
     return launch_dep(k_walk<D, MODE, COUNT, PER, POS_EPS, TEMP>, blocks < 1 ? 1 : blocks,
                       kWalkThreads, st, s, p, g, t, ie, inter, err);

@@ -104,18 +104,8 @@ k_key_levels(State s, StepParams p, Segs g, const uint64_t *__restrict__ keys, T
     const int64_t base = (int64_t)blockIdx.x * kKT;
     for (int q = threadIdx.x; q < kKT + 2 * kHalo + 1; q += kKT)
         sd[q] = (int8_t)delta_at<D>(g, keys, base - kHalo + q, n);
-    // parent child bits and counts are accumulated into pend by the emit pass
-    {
-        uint4 *p4 = reinterpret_cast<uint4 *>(t.pend);   // cudaMalloc: 16-byte aligned
-        const int64_t n4 = t.cap / 4;
-        for (int64_t k = (int64_t)blockIdx.x * kKT + threadIdx.x; k < n4;
-             k += (int64_t)gridDim.x * kKT)
-            p4[k] = make_uint4(0u, 0u, 0u, 0u);
-        if (blockIdx.x == 0 && threadIdx.x < (unsigned)(t.cap - n4 * 4))
-            t.pend[n4 * 4 + threadIdx.x] = 0u;
-        if (blockIdx.x == 0)
-            for (int q = threadIdx.x; q < kKeyBigHash; q += kKT) t.kbig_keys[q] = 0ull;
-    }
+    if (blockIdx.x == 0)
+        for (int q = threadIdx.x; q < kKeyBigHash; q += kKT) t.kbig_keys[q] = 0ull;
     // first levels whose cells are no larger than the size gate / min size
     // (the sizes are exact halvings of the root's: w * 2^-L)
     auto first_level_at_most = [&](float w, float limit) {
@@ -496,17 +486,16 @@ k_key_emit(State s, StepParams p, Segs g, const uint64_t *__restrict__ keys, Tre
                     L > 0 ? s_off[L - 1][w] + (uint32_t)__popc(s_bal[L - 1][w] & le) - 1u : kEmpty;
                 aux[4 * (size_t)slot + 0] = L;
                 aux[4 * (size_t)slot + 2] = parent;
-                aux[4 * (size_t)slot + 3] = L == X ? 1u : 0u;
+                const uint32_t dg = L > 0 ? digit<D>(key, (int)L - 1) : 0u;
+                aux[4 * (size_t)slot + 3] = (L == X ? 1u : 0u) | dg << kAuxDigit;
                 if (L > 0) {
-                    const uint32_t bit = 1u << digit<D>(key, (int)L - 1);
-                    atomicOr(&t.pend[parent], bit);
-                    // and in the tile's copy when the parent started in the tile
+                    // the child's bit in the tile's copy of its parent's mask,
+                    // when the parent started in the tile
                     const uint32_t pl = parent - s_off[L - 1][0];
                     if (parent >= s_off[L - 1][0] && pl < (uint32_t)kKT)
-                        atomicOr(&s_cm[L - 1][pl >> 2], bit << (8u * (pl & 3u)));
+                        atomicOr(&s_cm[L - 1][pl >> 2], (1u << dg) << (8u * (pl & 3u)));
                 }
                 if (L == X) {   // exact-rebuild roots have disjoint ranges: fewer than n
-                    atomicOr(&t.pend[slot], 1u << 31);
                     const uint32_t r = atomicAdd(&t.kmeta[kKmRoots], 1u);
                     if (r < n) t.kroots[r] = slot;
                 }
@@ -562,6 +551,7 @@ k_key_emit(State s, StepParams p, Segs g, const uint64_t *__restrict__ keys, Tre
     // 2; the build kernel combines the rest.  A node's children are the
     // contiguous level-(L+1) slots from its first child, in quadrant order. ----
     const uint32_t dl_next = w0 + kKT < n ? t.kdl[w0 + kKT] : 0u;
+    uint32_t partial = 0;   // levels at which this thread's node is left to the build kernel
     for (int L = (int)s_maxT; L >= 0; --L) {
         const uint32_t first = s_off[L][0], K = s_off[L][W] - first;
         if (K == 0u) continue;   // no node of this level starts in the tile
@@ -570,6 +560,7 @@ k_key_emit(State s, StepParams p, Segs g, const uint64_t *__restrict__ keys, Tre
             const uint32_t o = s_start[L][tid];   // tile index of the starting particle
             const uint32_t ww = o >> 5, ol = o & 31u;
             bool done = false;
+            uint32_t kids = 0;   // its children, once they are all known to be done
             float4 cm = make_float4(0.f, 0.f, 0.f, 0.f);
             const uint32_t ox = s_x[o];
             if ((uint32_t)L != ox) {
@@ -608,6 +599,7 @@ k_key_emit(State s, StepParams p, Segs g, const uint64_t *__restrict__ keys, Tre
                                 if (D == 3) c[2] = fdiv(c[2], gm);
                             }
                             cm = make_float4(c[0], c[1], c[2], gm);
+                            kids = mask;
                             done = true;
                         }
                     }
@@ -619,10 +611,38 @@ k_key_emit(State s, StepParams p, Segs g, const uint64_t *__restrict__ keys, Tre
                 // size at level L: the root's halved L times (exact)
                 const float szl = s_rs[o] * __int_as_float((127 - L) << 23);
                 put_walk<D>(t, slot, cm, szl);
-                aux[4 * (size_t)slot + 3] = 2u;
+                // done: its first byte, the digit beside it stays
+                reinterpret_cast<uint8_t *>(aux)[16 * (size_t)slot + 12] = 2u;
+            } else if ((uint32_t)L != ox) {
+                partial |= 1u << L;
             }
+            info[4 * (size_t)slot + 1] = kids;   // none yet: a leaf, an exact root, a partial node
         }
         __syncthreads();
+    }
+    // the partial nodes (across a tile's edge, or above an exact rebuild) are
+    // listed for the build kernel, which would otherwise look through all nodes
+    const uint32_t np = (uint32_t)__popc(partial);
+    uint32_t incl = np;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (unsigned)o) incl += u;
+    }
+    __shared__ uint32_t s_np[W], s_pbase;
+    if (lane == 31) s_np[w] = incl;
+    __syncthreads();
+    uint32_t before = 0, all = 0;
+#pragma unroll
+    for (int q = 0; q < W; q++) {
+        before += q < (int)w ? s_np[q] : 0u;
+        all += s_np[q];
+    }
+    if (tid == 0 && all) s_pbase = atomicAdd(&t.kmeta[kKmPartial], all);
+    __syncthreads();
+    if (np) {
+        uint32_t *to = partial_list(t) + s_pbase + before + incl - np;
+        for (uint32_t rest = partial; rest; rest &= rest - 1u) *to++ = s_off[__ffs(rest) - 1][0] + tid;
     }
 }
 

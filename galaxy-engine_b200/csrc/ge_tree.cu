@@ -1040,12 +1040,10 @@ k_build(State s, StepParams p, Segs g, Tree t, uint32_t *err, int keyed) {
     __shared__ __align__(16) unsigned char s_shared[kSharedBytes];
 
     // Keyed: the key passes (ge_kbuild.cu) wrote key_nodes nodes in slots
-    // [0, key_nodes), the segment roots first; pend holds each node's child
-    // bits (bit 31: an exact-rebuild root), aux.w marks exact-rebuild roots
-    // (1) and nodes whose mass is already final (2: every leaf, and the nodes
-    // inside one emit tile).  Phase 0 turns the bits into child masks and, for
-    // the other nodes, counts the children still pending; nodes with none are
-    // listed to be combined after the exact rebuilds (phases 1, 2).
+    // [0, key_nodes), the segment roots first, with their child masks and aux.w
+    // marks, and listed the partial ones.  Phase 0 gives those their masks and
+    // counts their children still pending; nodes with none are listed to be
+    // combined after the exact rebuilds (phases 1, 2).
     uint32_t lb = 0, le = (uint32_t)g.S, front = (uint32_t)g.S;
     uint32_t key_nodes = 0;   // keyed: slots [0, key_nodes) hold the key passes' nodes
     const uint32_t *list = nullptr;
@@ -1066,20 +1064,26 @@ k_build(State s, StepParams p, Segs g, Tree t, uint32_t *err, int keyed) {
     if (keyed) {
         key_nodes = *(volatile uint32_t *)&t.kmeta[3];
         if ((int64_t)key_nodes > t.cap) return;   // the emit pass set kErrNodeCap
-        for (uint32_t k = gtid; k < key_nodes; k += nthreads) {
-            const uint32_t pv = __ldcg(&t.pend[k]);
-            const uint32_t mask = pv & 0xFFu;
-            const bool exact = pv >> 31;
-            const bool done = __ldcg(&t.aux[k]).w & 2u;
-            reinterpret_cast<uint32_t *>(t.info)[4 * (size_t)k + 1] = exact ? 0u : mask;
-            uint32_t pending = 0;
-            if (!exact && !done) {
-                const uint32_t first = __ldcg(&t.info[k]).x;
-                const uint32_t nch = (uint32_t)__popc(mask);
-                for (uint32_t c = 0; c < nch; c++) pending += (__ldcg(&t.aux[first + c]).w & 2u) ? 0u : 1u;
+        // the partial nodes' child masks and pending counts, from their
+        // children (the contiguous slots from the first one that name it parent)
+        const uint32_t nparts = *(volatile uint32_t *)&t.kmeta[kKmPartial];
+        for (uint32_t q = gtid; q < nparts; q += nthreads) {
+            const uint32_t k = __ldcg(&partial_list(t)[q]);
+            const uint32_t first = __ldcg(&t.info[k]).x;
+            uint4 ca[1 << D];
+#pragma unroll
+            for (uint32_t c = 0; c < (1u << D); c++)
+                ca[c] = __ldcg(&t.aux[first + c < key_nodes ? first + c : first]);
+            uint32_t mask = 0, pending = 0;
+#pragma unroll
+            for (uint32_t c = 0; c < (1u << D); c++) {
+                if (first + c >= key_nodes || ca[c].z != k) continue;
+                mask |= 1u << ((ca[c].w >> kAuxDigit) & 7u);
+                pending += ca[c].w & 2u ? 0u : 1u;
             }
+            reinterpret_cast<uint32_t *>(t.info)[4 * (size_t)k + 1] = mask;
             t.pend[k] = pend_word(pending);
-            const bool ready = !exact && !done && pending == 0u;
+            const bool ready = pending == 0u;
             // combined after the exact rebuilds: list them (slot_of is free
             // until the layout)
             const unsigned lbits = __ballot_sync(__activemask(), ready);

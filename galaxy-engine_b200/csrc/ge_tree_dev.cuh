@@ -7,6 +7,17 @@
 
 namespace ge {
 
+// Key-prefix build: aux.w of a key node holds 1 for an exact-rebuild root, 2 for
+// a node whose mass is final, and its digit in its parent from bit kAuxDigit.
+// The nodes that are neither leaves, nor final, nor such roots are listed in
+// the walk layout's memory, which is free until the layout is written (at most
+// every node, in four times the words).
+constexpr int kAuxDigit = 8;
+constexpr int kKmPartial = 36;   // key meta word: partial nodes listed
+__device__ __forceinline__ uint32_t *partial_list(const Tree &t) {
+    return reinterpret_cast<uint32_t *>(t.src);
+}
+
 // std::partition_point(v + first, v + first + len, [mid](float a){ return a < mid; })
 // emulated by G consecutive lanes.  Lane j (1 <= j < G) of the group stands for
 // node j of the search's decision tree (heap order; child 2j when the probe is

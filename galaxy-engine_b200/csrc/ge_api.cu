@@ -1026,9 +1026,14 @@ int frame_overlapped(ge_ctx *c, int64_t n, const float *x, const float *y, const
             if ((rc = enqueue_walk(c, true))) return rc;
             GE_CHECK(c, back(0, n, s0));
         } else {
-            // the per-particle walk in particle ranges: each range's velocities and
-            // accelerations go back while the next range walks
-            constexpr int kParts = 4;
+            // the per-particle walk in up to four particle ranges: each range's
+            // velocities and accelerations go back while the next range walks.  A
+            // range too small to fill the chip walks hardly faster than a larger
+            // one, so small frames take one (frame in 2D by always four / by this
+            // rule, us: 20k 404 / 262, 140k 524 / 409, 262k 619 / 538, 600k 912 /
+            // 909; 3D, whose walks are longer, 70k 1058 / 562, 262k 1391 / 1064)
+            const int64_t range = D == 2 ? 131072 : 200000;
+            const int kParts = (int)std::max<int64_t>(1, std::min<int64_t>(4, n / range));
             StepParams p = step_params(c);
             State ws = cur_state(c);
             if (!c->p.temp_enabled) ws.temp = nullptr;

@@ -1408,7 +1408,7 @@ k_build(State s, StepParams p, Segs g, Tree t, uint32_t *err, int keyed) {
     // offset (the earlier chunks' total) is added where the scatter reads it:
     //   C(e) = endcnt[e] + s_boff[e / chunk]
     __shared__ uint32_t s_boff[kMaxBuildBlocks];
-    const uint32_t chunk = (n + 1 + gridDim.x - 1) / gridDim.x;
+    const uint32_t chunk = ((n + 1 + gridDim.x - 1) / gridDim.x + 3u) & ~3u;
     {
         constexpr int W = kBuildThreads / 32;
         __shared__ uint32_t s_w[W];
@@ -1416,10 +1416,19 @@ k_build(State s, StepParams p, Segs g, Tree t, uint32_t *err, int keyed) {
         const uint32_t c0 = min(blockIdx.x * chunk, total);
         const uint32_t c1 = min(c0 + chunk, total);
         uint32_t carry = 0;
-        for (uint32_t base = c0; base < c1; base += blockDim.x) {
-            const uint32_t i = base + threadIdx.x;
-            const uint32_t v = i < c1 ? __ldcg(&t.endcnt[i]) : 0u;
-            uint32_t incl = v;
+        // four counts per thread and round (chunks start at multiples of four)
+        for (uint32_t base = c0; base < c1; base += 4u * blockDim.x) {
+            const uint32_t i = base + 4u * threadIdx.x;
+            uint4 v = make_uint4(0u, 0u, 0u, 0u);
+            if (i + 3u < c1) {
+                v = __ldcg(reinterpret_cast<const uint4 *>(t.endcnt + i));
+            } else {
+                if (i < c1) v.x = __ldcg(&t.endcnt[i]);
+                if (i + 1u < c1) v.y = __ldcg(&t.endcnt[i + 1u]);
+                if (i + 2u < c1) v.z = __ldcg(&t.endcnt[i + 2u]);
+            }
+            v.y += v.x; v.z += v.y; v.w += v.z;
+            uint32_t incl = v.w;
             for (int o = 1; o < 32; o <<= 1) {
                 const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
                 if (lane >= (unsigned)o) incl += u;
@@ -1427,11 +1436,21 @@ k_build(State s, StepParams p, Segs g, Tree t, uint32_t *err, int keyed) {
             if (lane == 31) s_w[threadIdx.x >> 5] = incl;
             __syncthreads();
             uint32_t wpre = 0, btot = 0;
+#pragma unroll
             for (int w = 0; w < W; w++) {
-                if (w < (int)(threadIdx.x >> 5)) wpre += s_w[w];
-                btot += s_w[w];
+                const uint32_t x = s_w[w];
+                wpre += w < (int)(threadIdx.x >> 5) ? x : 0u;
+                btot += x;
             }
-            if (i < c1) t.endcnt[i] = carry + wpre + incl;
+            const uint32_t pre = carry + wpre + incl - v.w;
+            v.x += pre; v.y += pre; v.z += pre; v.w += pre;
+            if (i + 3u < c1) {
+                *reinterpret_cast<uint4 *>(t.endcnt + i) = v;
+            } else {
+                if (i < c1) t.endcnt[i] = v.x;
+                if (i + 1u < c1) t.endcnt[i + 1u] = v.y;
+                if (i + 2u < c1) t.endcnt[i + 2u] = v.z;
+            }
             carry += btot;
             __syncthreads();
         }

@@ -156,6 +156,8 @@ k_moments(State s, Tree t, double inv_theta, uint32_t *err) {
             // the children's masses and centres, then their moments, each in
             // one go (an absent child's load is the first one's again): a load
             // inside the sums is waited for there, a round trip per child
+            // (build stage with moments 1M 2D 342 -> 329 us, 100k 171 -> 139,
+            // 30k 3D 185 -> 126)
             double mc[Q], cc[Q][D];
 #pragma unroll
             for (int c = 0; c < Q; c++) {

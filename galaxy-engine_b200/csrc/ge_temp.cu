@@ -60,7 +60,8 @@ __global__ void __launch_bounds__(kTempThreads) k_node_temps(State s, Tree t) {
             if (pc.fetch_sub(1u, cuda::memory_order_acq_rel) != 1u) break;
             const uint4 pinf = __ldcg(&t.info[par]);
             // all children's sums first (an absent one's load is the first's
-            // again): a load inside the sum is waited for there
+            // again): a load inside the sum is waited for there (build stage of a
+            // 60k disk with heat exchange 147 -> 118 us)
             float ct[Q];
 #pragma unroll
             for (int q = 0; q < Q; q++) {

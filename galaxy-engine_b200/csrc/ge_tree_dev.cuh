@@ -11,7 +11,9 @@ namespace ge {
 // a node whose mass is final, and its digit in its parent from bit kAuxDigit.
 // The nodes that are neither leaves, nor final, nor such roots are listed in
 // the walk layout's memory, which is free until the layout is written (at most
-// every node, in four times the words).
+// every node, in four times the words).  (The children set their parents' bits
+// with global atomics before, and the build kernel looked through every node:
+// 1M step 799 -> 790 us, 96 small disks 387 -> 381.)
 constexpr int kAuxDigit = 8;
 constexpr int kKmPartial = 36;   // key meta word: partial nodes listed
 __device__ __forceinline__ uint32_t *partial_list(const Tree &t) {

@@ -108,7 +108,8 @@ typedef struct {
     float bbox[4];           /* last root box: x, y, (z,) size */
     float ms_last_step;      /* device time of the last ge_step call / nsteps */
     float stage_ms[8];       /* last ge_profile_step: kick+bbox, keys, sort, permute,
-                                build, walk, total, unused */
+                                build, walk, total, unused (small simulations: one
+                                launch for the first four, its time under kick+bbox) */
 } ge_stats;
 
 typedef struct ge_ctx ge_ctx;

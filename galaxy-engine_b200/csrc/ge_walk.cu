@@ -39,11 +39,22 @@
 namespace ge {
 
 // Threads per block: a block's particles, consecutive in Morton order on one
-// SM, share most of their walks through L1, so small systems take no smaller
-// blocks (16k in 2D: 51 us, 59 with 64 threads).  (1024 in 3D shared more while
-// a link had 8 bytes, 1M 1.65 ms against 1.78; with packed links 256 takes
-// 1.56, 250k 483 us against 537, 60k 188 against 275, 16k 142 against 227.)
-constexpr int kWalkThreads = 256;
+// SM, share most of their walks through L1.  (1024 in 3D shared more while a
+// link had 8 bytes, 1M 1.65 ms against 1.78; with packed links 256 takes 1.56,
+// 250k 483 us against 537, 60k 188 against 275, 16k 142 against 227.)
+constexpr int kWalkThreads = 256, kWalkThreads2D = 512;
+// 2D, by the launch's particles.  While SMs are left over, larger blocks share
+// more (256 -> 512 threads, us: 2k 38.9 -> 36.8, 6k 49.2 -> 45.1, 12k 53.3 ->
+// 49.2, 20k 55.3 -> 53.8, 28k 55.8 -> 54.3, 36k the same; with heat exchange 12k
+// 133 -> 126).  Between one and four blocks of 256 per SM some SMs have one more
+// than others, which smaller blocks even out (256 -> 128: 45k 57.3 -> 55.3, 65k
+// 57.3 -> 53.2, 90k 57.5 -> 55.3, 130k 56.7 -> 55.3; with heat exchange 65k 139 ->
+// 131; 36k the same, 190k 65.5 -> 66.6).  3D gains on neither side (20k 157.7,
+// 159.7 with 512; 65k 178.2, 181.7 with 128).
+static int walk_threads_2d(int n) {
+    constexpr int kSms = 148;
+    return n <= 64 * 512 ? 512 : n > kSms * 256 && n <= 4 * kSms * 256 ? 128 : 256;
+}
 
 __device__ __forceinline__ float wrap_d(float d, float dom, float hd) {
     // d -= domain * ((d > half) - (d < -half))   (physics.cpp:118-121), the
@@ -121,7 +132,7 @@ __device__ __forceinline__ void walk_packed2(const float4 *__restrict__ src, uin
 }
 
 template <int D, int MODE, bool COUNT, bool PER, bool POS_EPS, bool TEMP = false>
-__global__ void __launch_bounds__(kWalkThreads)
+__global__ void __launch_bounds__(D == 2 ? kWalkThreads2D : kWalkThreads)
 k_walk(State s, StepParams p, Segs g, Tree t, int integrate_end, unsigned long long *inter,
        uint32_t *err) {
     dep_wait();
@@ -503,9 +514,11 @@ static cudaError_t walk_one(const State &s, const StepParams &p, const Segs &g, 
         if (walk_pairs(p))
             return launch_dep(k_walk_pair<PER>, (p.n - p.i0 + 2 * kPairThreads - 1) / (2 * kPairThreads),
                               kPairThreads, st, s, p, g, t, ie);
-    const int blocks = (p.n - p.i0 + kWalkThreads - 1) / kWalkThreads;
+    // (the mixed mode's per-particle form was not measured and stays at 256)
+    const int threads = D == 2 && MODE != GE_PREC_MIXED ? walk_threads_2d(p.n - p.i0) : kWalkThreads;
+    const int blocks = (p.n - p.i0 + threads - 1) / threads;
     return launch_dep(k_walk<D, MODE, COUNT, PER, POS_EPS, TEMP>, blocks < 1 ? 1 : blocks,
-                      kWalkThreads, st, s, p, g, t, ie, inter, err);
+                      threads, st, s, p, g, t, ie, inter, err);
 }
 
 template <int D, int MODE, bool PER>

@@ -129,6 +129,7 @@ struct ge_ctx {
     std::vector<uint8_t> h_dflag;
     bool any_direct = false, any_walk = true;
     int front = 0;                // front_plan of the current simulations
+    FrontLimits front_lim[2];     // 2D, 3D: this context's device
     uint32_t *d_err = nullptr;
     uint32_t *h_meta = nullptr;   // pinned copy of the tree meta words
     int64_t slots = 0;            // node slots of the last build (holes included)
@@ -629,7 +630,7 @@ int sync_segments(ge_ctx *c) {
     c->b.ss.box_blocks = (int)bb;
     int64_t largest = 0;
     for (const SimRec &s : c->sims) largest = std::max(largest, s.n);
-    c->front = front_plan(c->p.dims, largest, S);
+    c->front = front_plan(c->p.dims, largest, S, c->front_lim[c->p.dims == 2 ? 0 : 1]);
     c->tree_valid = false;
     c->keys_valid = false;
     return direct_tables(c);

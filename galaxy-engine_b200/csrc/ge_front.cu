@@ -28,9 +28,8 @@ namespace ge {
 
 constexpr int kFrontThreads = 512;
 constexpr int kFrontWarps = kFrontThreads / 32;
-constexpr uint32_t kFrontCluster = 16;   // most blocks per simulation
+constexpr uint32_t kFrontCluster = 1u << (kFrontSizes - 1);   // most blocks per simulation: 16
 constexpr int kFrontItems = 4;           // most particles per thread
-constexpr int kFrontWave = 2 * 148;      // blocks that are resident together
 constexpr int kFrontBits = 9, kFrontRadix = 1 << kFrontBits;   // as the per-pass sort
 static_assert(kFrontRadix == kFrontThreads, "one thread per digit");
 
@@ -252,61 +251,79 @@ static cudaError_t front_launch(int blocks, int cluster, cudaStream_t st, const 
     return cudaLaunchKernelEx(&cfg, k_front<D, ITEMS>, in, out, p, g, t, ss.keys[0], ss.vals[0]);
 }
 
-// Once per kernel and process: more than 48 KB of shared memory and, where the
-// device can hold one, clusters of 16 blocks.  Largest usable cluster, 0: none.
+// More than 48 KB of shared memory and clusters of 16 blocks (a device that
+// refuses those keeps the 8 that every device has).  Both are attributes of the
+// kernel on the current device.
 template <int D, int ITEMS>
-static int front_setup() {
+static bool front_attributes() {
     const void *k = (const void *)k_front<D, ITEMS>;
-    const int bytes = (int)sizeof(FrontSmem<D, ITEMS>);
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) {
+    const bool ok = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)sizeof(FrontSmem<D, ITEMS>)) == cudaSuccess;
+    if (!ok || cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
         (void)cudaGetLastError();
-        return 0;
-    }
-    const bool np = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
-                    cudaSuccess;
-    if (!np) (void)cudaGetLastError();
-    for (int c = np ? (int)kFrontCluster : 8; c >= 1; c /= 2) {
+    return ok;
+}
+
+template <int D>
+static void front_limits(FrontLimits &lim) {
+    lim.known = true;
+    if (!front_attributes<D, 1>() || !front_attributes<D, 2>() || !front_attributes<D, 4>()) return;
+    for (int q = 0; q < kFrontSizes; q++) {   // the variant with the most shared memory
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(c);
+        cfg.gridDim = dim3(1u << q);
         cfg.blockDim = dim3(kFrontThreads);
-        cfg.dynamicSmemBytes = bytes;
+        cfg.dynamicSmemBytes = sizeof(FrontSmem<D, kFrontItems>);
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = (unsigned)c;
+        attr[0].val.clusterDim.x = 1u << q;
         attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         int fit = 0;
-        if (cudaOccupancyMaxActiveClusters(&fit, k, &cfg) == cudaSuccess && fit > 0) return c;
-        (void)cudaGetLastError();
+        if (cudaOccupancyMaxActiveClusters(&fit, (const void *)k_front<D, kFrontItems>, &cfg) !=
+            cudaSuccess) {
+            (void)cudaGetLastError();
+            fit = 0;
+        }
+        lim.fit[q] = fit;
     }
-    return 0;
-}
-
-template <int D>
-static int front_limit() {   // the largest cluster every variant can use
-    static const int lim = min(min(front_setup<D, 1>(), front_setup<D, 2>()), front_setup<D, 4>());
-    return lim;
 }
 
 // Few keys per block keep a pass short, many blocks make its barriers and
 // remote stores long (a pass at 16 blocks: 0.7 us of ranking, 2 us for the
-// counts, 1.8 us for the keys).  Step time against the per-pass kernels (us):
+// counts, 1.8 us for the keys), and a second block on an SM costs as much as
+// the shorter passes gain (10 simulations of 16k in clusters of 16 blocks: kick
+// to gather 55 us, of 8 blocks 43).  So: the largest cluster that holds every
+// simulation with one block per SM (half of those that fit, which are fewer
+// than the SMs allow: a cluster lies inside one GPC, 14 of 16 blocks, 33 of 8,
+// 71 of 4).  Where none does, the smallest that holds the largest simulation,
+// while at most an eighth more of them than fit wait for the first to end and
+// there are no more blocks than fit one by one; else the per-pass kernels.
+// Step against those (us):
 //   2D 2k 174 -> 154, 16k 179 -> 162, 32k 186 -> 177, 45k 189 -> 193 (8 items)
 //   3D 16k 391 -> 356, 60k 465 -> 473
-//   100 simulations of up to 4k 220 -> 208, 16 of up to 16k 187 -> 187
-// so up to 32,768 particles each, while every block is resident at once (96
-// simulations of up to 16k in three waves: 359 -> 374).
-int front_plan(int dims, int64_t largest, int64_t sims) {
-    const int lim = dims == 2 ? front_limit<2>() : front_limit<3>();
-    if (sims < 1 || lim < 1) return 0;
-    int c = 1;
-    while (c < lim && (int64_t)c * kFrontThreads < largest) c *= 2;
-    while (c > 1 && sims * c > kFrontWave) c /= 2;
-    if (sims * c > kFrontWave || (int64_t)c * kFrontThreads * kFrontItems < largest) return 0;
+//   2D, 10 of 16k in clusters of 16 / 8 blocks 172 / 159 (per pass 179), 18
+//   220 / 203 (218); 72 of 4k in clusters of 4 / 2 190 / 175 (210); 73 of up to
+//   8k in clusters of 4 224 (231), 35 of up to 16k of 8 215 (220); 16 of up to
+//   32k in clusters of 16 194 (192), 18 217 (205)
+int front_plan(int dims, int64_t largest, int64_t sims, FrontLimits &lim) {
+    if (sims < 1 || largest > (int64_t)kFrontCluster * kFrontThreads * kFrontItems) return 0;
+    if (!lim.known) {
+        if (dims == 2) front_limits<2>(lim);
+        else front_limits<3>(lim);
+    }
+    int best = -1;   // log2 of the blocks
+    for (int q = kFrontSizes - 1; q >= 0; q--) {
+        const int64_t threads = (int64_t)kFrontThreads << q;
+        if (threads * kFrontItems < largest) break;
+        if (q > 0 && threads / 2 >= largest) continue;   // half of it would do
+        if (sims <= lim.fit[q] + lim.fit[q] / 8 && sims << q <= lim.fit[0]) best = q;
+        if (2 * sims <= lim.fit[q]) break;
+    }
+    if (best < 0) return 0;
     int items = 1;
-    while ((int64_t)items * kFrontThreads * c < largest) items *= 2;
-    return c << 8 | items;
+    while (((int64_t)items * kFrontThreads << best) < largest) items *= 2;
+    return 256 << best | items;
 }
 
 template <int D>

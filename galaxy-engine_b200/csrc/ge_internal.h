@@ -321,8 +321,14 @@ cudaError_t launch_permute(int dims, int n, const SortScratch &ss, const State &
 // kick + drift, box, keys, sort and gather of every segment in one launch
 // (ge_front.cu), the state moving from `in` to `out`.  plan: what front_plan
 // chose for the largest segment's size and the number of segments (0: some
-// segment is too large for it, the passes run one by one).
-int front_plan(int dims, int64_t largest, int64_t sims);
+// segment is too large for it or they are too many, the passes run one by one).
+// lim: what the context's device can hold, filled when a plan first needs it.
+constexpr int kFrontSizes = 5;   // clusters of 1, 2, 4, 8, 16 blocks
+struct FrontLimits {
+    bool known = false;
+    int fit[kFrontSizes] = {};   // clusters of 2^k blocks resident together (0: none)
+};
+int front_plan(int dims, int64_t largest, int64_t sims, FrontLimits &lim);
 cudaError_t launch_front(int dims, int plan, const State &in, const State &out,
                          const StepParams &p, const Segs &g, const Tree &t, SortScratch &ss,
                          cudaStream_t st);

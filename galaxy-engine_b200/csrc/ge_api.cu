@@ -911,6 +911,11 @@ int get_host(ge_ctx *c, int64_t off, int64_t n, float *x, float *y, float *z, fl
         {m, s.m + off, B}, {id, s.id + off, sizeof(uint32_t) * (size_t)n}};
     HostArrays h{};
     bool direct = n <= kStoreMax;
+    // arrays that share memory are written one after another: the last one wins
+    for (auto &q : cp)
+        for (auto *o = cp; o != &q; o++)
+            direct = direct && !(q.h && o->h && static_cast<char *>(q.h) < static_cast<char *>(o->h) + o->b &&
+                                 static_cast<char *>(o->h) < static_cast<char *>(q.h) + q.b);
     for (auto &q : cp) {
         if (!q.h || !direct) continue;
         uint32_t *dst = static_cast<uint32_t *>(page_locked(q.h, q.b));

@@ -224,7 +224,10 @@ constexpr int kMetaWalkPacked = 13;
 // (the warp-cooperative walk reads it)
 constexpr int kLayoutEntry = 1, kLayoutRange = 2;
 constexpr int kMetaBigRoot = 14;   // tree meta word: some simulation's root size >= 1e19
-constexpr int kMetaNegMass = 17;   // tree meta word: some mass is negative (centres may leave the box)
+// tree meta word: a mass is negative or, in a periodic domain, something with
+// mass lies outside its root box by more than kBoxSlack of half the domain
+constexpr int kMetaMayWrap = 17;
+constexpr float kBoxSlack = 0.049f;
 constexpr int kMetaWords = 32;     // tree meta words allocated
 // warp-cooperative walk counters (Tree::wctr, zeroed before each launch): the
 // chunk counter and the count of chunks that fell back to the per-particle walk

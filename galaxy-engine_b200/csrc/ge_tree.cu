@@ -948,25 +948,43 @@ __device__ bool build_small_subtree_smem(const State &s, const StepParams &p, Tr
 // The walk-layout entries of node slot k (and of its particles when it is a
 // leaf), from its fields and the end counts C(start) = ez, C(end) = ew.
 template <int D>
-__device__ __forceinline__ void scatter_entry(const State &s, const Segs &g, Tree &t, uint32_t k,
-                                              uint4 inf, uint4 ax, float4 w, float size2,
+__device__ __forceinline__ void scatter_entry(const State &s, const StepParams &p, const Segs &g,
+                                              Tree &t, uint32_t k, uint4 inf, uint4 ax, float4 w, float size2,
                                               uint32_t ez, uint32_t ew, uint32_t total,
-                                              uint32_t *err, bool packed, int extras) {
+                                              uint32_t *err, bool packed) {
     const uint32_t me = ez + ax.x + inf.z;
     const uint32_t skip = ew + ax.x - ax.y + inf.w;
     if (me >= total || skip > total) {   // cannot happen for a consistent tree
         set_err(err, kErrDepth);
         return;
     }
-    if (extras & kLayoutEntry) t.aux[k].w = me;   // the node's entry
-    if (extras & kLayoutRange) t.nrange[k] = make_uint2(me, skip);   // its layout range
+    if (p.layout_extras & kLayoutEntry) t.aux[k].w = me;   // the node's entry
+    if (p.layout_extras & kLayoutRange) t.nrange[k] = make_uint2(me, skip);   // its layout range
     if (k < (uint32_t)g.S) {   // a segment's root: where its particles' walks start and end
         g.root_begin[k] = me;
         g.root_end[k] = skip;
     }
     const float nm = D == 2 ? w.z : w.w;
     const bool massless = nm <= 0.0f;
-    bool negative = nm < 0.0f;
+    // the periodic walk leaves the wrap out only while everything it can meet
+    // lies in the root box up to kBoxSlack (never_wraps): a leaf's plain sums
+    // drift with its particles, and negative masses throw a centre anywhere
+    bool outside = nm < 0.0f;
+    float4 box = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto beyond = [&](float x, float y, float z) {
+        const float v[3] = {x, y, z}, lo[3] = {box.x, box.y, box.z};
+        bool in = true;
+#pragma unroll
+        for (int a = 0; a < D; a++) {
+            const float slack = kBoxSlack * p.half_domain[a];
+            in = in && v[a] >= lo[a] - slack && v[a] <= lo[a] + box.w + slack;
+        }
+        return !in;
+    };
+    if (p.periodic) {
+        box = g.box[g.seg_of ? g.seg_of[inf.z] : 0u];
+        outside = outside || (!massless && beyond(w.x, w.y, w.z));
+    }
     if (massless) {
         // gridMass <= 0: the reference skips the whole subtree.  As a source
         // it is accepted by every test (size^2 = -2; particles have -1),
@@ -986,7 +1004,7 @@ __device__ __forceinline__ void scatter_entry(const State &s, const Segs &g, Tre
         else if (!packed) ((uint32_t *)t.link)[me] = skip;
     }
     if (inf.y) {
-        if (negative) t.meta[kMetaNegMass] = 1u;
+        if (outside) t.meta[kMetaMayWrap] = 1u;
         return;
     }
     // a leaf: its particles follow it, four at a time (loads before stores)
@@ -1000,7 +1018,7 @@ __device__ __forceinline__ void scatter_entry(const State &s, const Segs &g, Tre
             py[q] = in ? s.y[j] : 0.0f;
             pz[q] = in && D == 3 ? s.z[j] : 0.0f;
             pm[q] = in ? s.m[j] : 0.0f;
-            negative = negative || pm[q] < 0.0f;
+            outside = outside || pm[q] < 0.0f || (in && p.periodic && beyond(px[q], py[q], pz[q]));
         }
 #pragma unroll
         for (int q = 0; q < 4; q++) {
@@ -1021,7 +1039,7 @@ __device__ __forceinline__ void scatter_entry(const State &s, const Segs &g, Tre
             }
         }
     }
-    if (negative) t.meta[kMetaNegMass] = 1u;
+    if (outside) t.meta[kMetaMayWrap] = 1u;
 }
 
 template <int D>
@@ -1054,7 +1072,7 @@ k_build(State s, StepParams p, Segs g, Tree t, uint32_t *err, int keyed) {
         t.meta[kMetaNodes] = 0u; t.meta[kMetaLevels] = 0u;
         t.meta[kMetaSmall] = 0u; t.meta[kMetaP2Alloc] = 0u; t.meta[kMetaTimeline] = 0u;
         t.meta[kMetaReal] = 0u; t.meta[kMetaSlots] = 0u; t.meta[kMetaP2Task] = 0u;
-        t.meta[kMetaBigRoot] = 0u; t.meta[kMetaNegMass] = 0u; t.meta[kMetaDone] = 0u; t.kmeta[kKmProdDone] = 0u;
+        t.meta[kMetaBigRoot] = 0u; t.meta[kMetaMayWrap] = 0u; t.meta[kMetaDone] = 0u; t.kmeta[kKmProdDone] = 0u;
         const uint32_t id = t.meta[kMetaBuildId] + 1u;   // read after the first grid barrier
         t.meta[kMetaBuildId] = id ? id : 1u;
         stamp(t);
@@ -1528,8 +1546,8 @@ k_build(State s, StepParams p, Segs g, Tree t, uint32_t *err, int keyed) {
 #pragma unroll
         for (int u = 0; u < 2; u++) {
             if (inf[u].w == 0u) continue;
-            scatter_entry<D>(s, g, t, kk[u], inf[u], ax[u], wv[u], s2[u], ez[u], ew[u], total, err,
-                             packed, p.layout_extras);
+            scatter_entry<D>(s, p, g, t, kk[u], inf[u], ax[u], wv[u], s2[u], ez[u], ew[u], total, err,
+                             packed);
         }
     }
     // the last block to finish stamps the end of the build

@@ -64,17 +64,18 @@ __device__ __forceinline__ float wrap_d(float d, float dom, float hd) {
 }
 
 // Whether no offset from a particle to anything inside its simulation's root
-// box can pass half the domain, so that the wrap leaves every offset as it is.
-// Centres of mass lie in the box when no mass is negative, up to their sums'
-// rounding: the margin (5 % of half the domain, coordinates up to twice the
-// domain) covers plain sums of 10^5 coincident particles.  In a 3D sphere of
-// 250k reaching 77 % of the domain this holds for most particles: walk 566 ->
-// 477 us; a 2D disk of 1M well inside it 421 -> 271 (no wrap at all: 271).
+// box can pass half the domain, so that the wrap leaves every offset as it is:
+// the particle has 0.95 of half the domain to the box's sides, and the build
+// has seen nothing farther outside the box than kBoxSlack (0.049) of it; the
+// thousandth between them is for the roundings (coordinates up to twice the
+// domain).  In a 3D sphere of 250k reaching 77 % of the domain this holds for
+// most particles: walk 566 -> 477 us; a 2D disk of 1M well inside it 421 -> 271
+// (no wrap at all: 271).
 template <int D>
 __device__ __forceinline__ bool never_wraps(const Tree &t, const float4 &box, const StepParams &p,
                                             const float *x) {
     const float lo[3] = {box.x, box.y, box.z};
-    bool in = __ldg(&t.meta[kMetaNegMass]) == 0u;
+    bool in = __ldg(&t.meta[kMetaMayWrap]) == 0u;
 #pragma unroll
     for (int a = 0; a < D; a++) {
         const float most = 0.95f * p.half_domain[a];

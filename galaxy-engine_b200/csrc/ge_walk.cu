@@ -301,8 +301,11 @@ k_walk(State s, StepParams p, Segs g, Tree t, int integrate_end, unsigned long l
                 else k = max(k + 1, acc && !part ? nxt_skip : k + 1);
             }
         };
-        // a periodic walk whose offsets cannot wrap is the plain one
-        const bool wraps = PER && !never_wraps<D>(t, g.box[sg], p, pi);
+        // a periodic walk whose offsets cannot wrap is the plain one; a warp that
+        // holds both kinds of particles wraps for all (the same bits) instead of
+        // running both loops one after the other
+        const bool wraps =
+            PER && __any_sync(__activemask(), !never_wraps<D>(t, g.box[sg], p, pi));
         if constexpr (!kSelfTest && D == 2) {
             // As signed words the size^2 of a node and theta^2 r2 compare as
             // the floats do, and a marker level (62 or 63 off the root's
@@ -484,6 +487,7 @@ k_walk_pair(State s, StepParams p, Segs g, Tree t, int integrate_end) {
                 const float x[3] = {s.x[i[q]], s.y[i[q]], pz[q]};
                 wraps = wraps || !never_wraps<3>(t, g.box[sgp], p, x);
             }
+        if (PER) wraps = __any_sync(__activemask(), wraps);   // as in the single walk
         if constexpr (PER) {
             if (wraps) by_layout(std::true_type{});
             else by_layout(std::false_type{});

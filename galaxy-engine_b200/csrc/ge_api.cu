@@ -704,7 +704,8 @@ int enqueue_build(ge_ctx *c, bool fresh_keys = false) {
     // the optional layout arrays this build's readers need
     const bool temps = c->p.temp_enabled && c->b.temp;
     p.layout_extras = (c->p.precision == GE_PREC_MIXED || temps ? kLayoutEntry : 0) |
-                      (c->p.walk_kind == 1 ? kLayoutRange : 0);
+                      (c->p.walk_kind == 1 ? kLayoutRange : 0) |
+                      (c->p.dims == 3 && temps ? kLayoutPlain : 0);
     c->tree_ranges = c->p.walk_kind == 1;
     const bool keyed = fresh_keys && c->p.leaf_cap >= 1 && c->p.leaf_cap <= (uint32_t)kKeyMaxCap;
     if (keyed)

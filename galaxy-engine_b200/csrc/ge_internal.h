@@ -204,7 +204,7 @@ struct StepParams {
     int i0;              // the per-particle walk: first particle (up to n), 0 by default
     int mixed;           // GE_PREC_MIXED: the moment pass rewrites the node entries
     int walk_kind;       // GE_PREC_FAST: 0 per-particle walk, 1 warp-cooperative walk
-    int layout_extras;   // tree build: kLayoutEntry | kLayoutRange (the optional layout arrays)
+    int layout_extras;   // tree build: kLayoutEntry | kLayoutRange (the optional layout arrays) | kLayoutPlain
 };
 
 // 2D walk entries {x, y, m, w}.  Plain layout: w = size^2 (-1 for a particle,
@@ -223,6 +223,12 @@ constexpr int kMetaWalkPacked = 13;
 // moment and node-temperature passes read it) and its entry range in nrange
 // (the warp-cooperative walk reads it)
 constexpr int kLayoutEntry = 1, kLayoutRange = 2;
+// the plain layout whatever the sizes allow.  3D walks with heat exchange read
+// it: their steps hang on the chain through the temperature, not on the loads
+// that packed words save, and unpacking them lengthens it (walk, packed / plain,
+// us: 5k 315 / 293, 100k 554 / 522, 300k 1078 / 994, 700k 2343 / 2275; EXACT 300k
+// 1561 / 1464; without heat exchange 300k 445 / 637)
+constexpr int kLayoutPlain = 4;
 constexpr int kMetaBigRoot = 14;   // tree meta word: some simulation's root size >= 1e19
 // tree meta word: a mass is negative or, in a periodic domain, something with
 // mass lies outside its root box by more than kBoxSlack of half the domain

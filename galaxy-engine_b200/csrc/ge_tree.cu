@@ -1513,12 +1513,12 @@ k_build(State s, StepParams p, Segs g, Tree t, uint32_t *err, int keyed) {
     //   subtree successor    = C(end) + level - same_end + end
     //   entry of particle j  = entry of its leaf + 1 + (j - start)
     const uint32_t total = nodes + n;
-    // unless the moment pass rewrites them: packed entries when every level
-    // and successor fits the word and every size^2 is a normal float (a node
-    // of size <= min_size is a leaf, so sizes stay >= min_size / 2, or the
-    // tree is one leaf; root sizes below 1e19), where quartering L times is
-    // the exponent minus 2L
-    const bool packed = !p.mixed && p.min_size >= 1e-18f &&
+    // unless the moment pass rewrites them or their walk wants them plain: packed
+    // entries when every level and successor fits the word and every size^2 is
+    // a normal float (a node of size <= min_size is a leaf, so sizes stay >=
+    // min_size / 2, or the tree is one leaf; root sizes below 1e19), where
+    // quartering L times is the exponent minus 2L
+    const bool packed = !p.mixed && !(p.layout_extras & kLayoutPlain) && p.min_size >= 1e-18f &&
                         *(volatile uint32_t *)&t.meta[kMetaBigRoot] == 0u &&
                         *(volatile uint32_t *)&t.meta[kMetaLevels] <= kPackMaxLevel + 1u &&
                         total < (1u << kPackSkipBits);

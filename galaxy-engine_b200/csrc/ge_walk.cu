@@ -42,7 +42,22 @@ namespace ge {
 // SM, share most of their walks through L1.  (1024 in 3D shared more while a
 // link had 8 bytes, 1M 1.65 ms against 1.78; with packed links 256 takes 1.56,
 // 250k 483 us against 537, 60k 188 against 275, 16k 142 against 227.)
-constexpr int kWalkThreads = 256, kWalkThreads2D = 512;
+constexpr int kWalkThreads = 256, kWalkThreads2D = 512, kWalkThreadsRows = 1024;
+// 3D EXACT, MIXED and heat exchange: blocks of 1024 share more still, and take
+// less time where their last row (one block on every SM) is at least nine tenths
+// full; with a row that is not, the SMs with one block more than others cost more
+// than the sharing gains.  Walk, 256 / 1024 threads (us): EXACT 150k 394 / 390, 160k
+// 464 / 607, 300k 773 / 710, 350k 955 / 1007, 450k 1127 / 1078, 605k 1451 / 1402, 1M
+// 2355 / 2352; with heat exchange 300k 1489 / 1362; FAST with heat exchange 300k 1008
+// / 942, 450k 1530 / 1538, 605k 1914 / 1817.  MIXED takes 38 registers with 256
+// threads (faster below its six blocks per SM: 50k 672 / 1057) and 32 with 1024,
+// where a row alone on the SMs is slow, so two rows have to be full: 285k 3205 /
+// 2365, 300k 3141 / 2483, 450k 3707 / 4164, 605k 5161 / 4670, 900k 7356 / 6928.
+static bool walk_rows_full(int mode, int n, int num_sms) {
+    const int row = mode == GE_PREC_MIXED ? 2 * num_sms : num_sms;
+    const int last = ((n + kWalkThreadsRows - 1) / kWalkThreadsRows - 1) % row + 1;
+    return n > 0 && 10 * last >= 9 * row;
+}
 // 2D, by the launch's particles.  While SMs are left over, larger blocks share
 // more (256 -> 512 threads, us: 2k 38.9 -> 36.8, 6k 49.2 -> 45.1, 12k 53.3 ->
 // 49.2, 20k 55.3 -> 53.8, 28k 55.8 -> 54.3, 36k the same; with heat exchange 12k
@@ -132,8 +147,13 @@ __device__ __forceinline__ void walk_packed2(const float4 *__restrict__ src, uin
     unpack2(fxy, f[0], f[1]);
 }
 
-template <int D, int MODE, bool COUNT, bool PER, bool POS_EPS, bool TEMP = false>
-__global__ void __launch_bounds__(D == 2 ? kWalkThreads2D : kWalkThreads)
+// 0: the compiler's choice
+constexpr int walk_min_blocks(int dims, int mode, int threads) {
+    return dims == 2 || (mode == GE_PREC_MIXED && threads == kWalkThreads) ? 0 : 2048 / threads;
+}
+
+template <int D, int MODE, bool COUNT, bool PER, bool POS_EPS, bool TEMP, int THREADS>
+__global__ void __launch_bounds__(THREADS, walk_min_blocks(D, MODE, THREADS))
 k_walk(State s, StepParams p, Segs g, Tree t, int integrate_end, unsigned long long *inter,
        uint32_t *err) {
     dep_wait();
@@ -514,38 +534,52 @@ k_walk_pair(State s, StepParams p, Segs g, Tree t, int integrate_end) {
 
 template <int D, int MODE, bool COUNT, bool PER, bool POS_EPS, bool TEMP = false>
 static cudaError_t walk_one(const State &s, const StepParams &p, const Segs &g, const Tree &t,
-                            int ie, unsigned long long *inter, uint32_t *err, cudaStream_t st) {
+                            int ie, unsigned long long *inter, uint32_t *err, int num_sms,
+                            cudaStream_t st) {
     if constexpr (D == 3 && MODE == GE_PREC_FAST && !COUNT && POS_EPS && !TEMP)
         if (walk_pairs(p))
             return launch_dep(k_walk_pair<PER>, (p.n - p.i0 + 2 * kPairThreads - 1) / (2 * kPairThreads),
                               kPairThreads, st, s, p, g, t, ie);
-    // (the mixed mode's per-particle form was not measured and stays at 256)
-    const int threads = D == 2 && MODE != GE_PREC_MIXED ? walk_threads_2d(p.n - p.i0) : kWalkThreads;
-    const int blocks = (p.n - p.i0 + threads - 1) / threads;
-    return launch_dep(k_walk<D, MODE, COUNT, PER, POS_EPS, TEMP>, blocks < 1 ? 1 : blocks,
-                      threads, st, s, p, g, t, ie, inter, err);
+    const int n = p.n - p.i0;
+    auto go = [&](auto bound, int threads) {
+        const int blocks = (n + threads - 1) / threads;
+        return launch_dep(k_walk<D, MODE, COUNT, PER, POS_EPS, TEMP, decltype(bound)::value>,
+                          blocks < 1 ? 1 : blocks, threads, st, s, p, g, t, ie, inter, err);
+    };
+    if constexpr (D == 2) {
+        return go(std::integral_constant<int, kWalkThreads2D>{},
+                  MODE != GE_PREC_MIXED ? walk_threads_2d(n) : kWalkThreads);
+    } else {
+        if constexpr (MODE != GE_PREC_FAST || TEMP)
+            if (walk_rows_full(MODE, n, num_sms))
+                return go(std::integral_constant<int, kWalkThreadsRows>{}, kWalkThreadsRows);
+        return go(std::integral_constant<int, kWalkThreads>{}, kWalkThreads);
+    }
 }
 
 template <int D, int MODE, bool PER>
 static cudaError_t walk_eps(const State &s, const StepParams &p, const Segs &g, const Tree &t,
-                            int ie, unsigned long long *inter, uint32_t *err, cudaStream_t st) {
+                            int ie, unsigned long long *inter, uint32_t *err, int num_sms,
+                            cudaStream_t st) {
     if constexpr (MODE != GE_PREC_MIXED)
         if (s.temp && t.tv) {   // heat exchange (counting included)
-            if (inter) return walk_one<D, MODE, true, PER, false, true>(s, p, g, t, ie, inter, err, st);
-            return walk_one<D, MODE, false, PER, false, true>(s, p, g, t, ie, nullptr, err, st);
+            if (inter)
+                return walk_one<D, MODE, true, PER, false, true>(s, p, g, t, ie, inter, err, num_sms, st);
+            return walk_one<D, MODE, false, PER, false, true>(s, p, g, t, ie, nullptr, err, num_sms, st);
         }
-    if (inter) return walk_one<D, MODE, true, PER, false>(s, p, g, t, ie, inter, err, st);
+    if (inter) return walk_one<D, MODE, true, PER, false>(s, p, g, t, ie, inter, err, num_sms, st);
     if constexpr (MODE != GE_PREC_MIXED)   // MIXED always tests for the particle itself
         if (p.eps2 > 0.0f)
-            return walk_one<D, MODE, false, PER, true>(s, p, g, t, ie, nullptr, err, st);
-    return walk_one<D, MODE, false, PER, false>(s, p, g, t, ie, nullptr, err, st);
+            return walk_one<D, MODE, false, PER, true>(s, p, g, t, ie, nullptr, err, num_sms, st);
+    return walk_one<D, MODE, false, PER, false>(s, p, g, t, ie, nullptr, err, num_sms, st);
 }
 
 template <int D, int MODE>
 static cudaError_t walk_mode(const State &s, const StepParams &p, const Segs &g, const Tree &t,
-                             int ie, unsigned long long *inter, uint32_t *err, cudaStream_t st) {
-    if (p.periodic) return walk_eps<D, MODE, true>(s, p, g, t, ie, inter, err, st);
-    return walk_eps<D, MODE, false>(s, p, g, t, ie, inter, err, st);
+                             int ie, unsigned long long *inter, uint32_t *err, int num_sms,
+                            cudaStream_t st) {
+    if (p.periodic) return walk_eps<D, MODE, true>(s, p, g, t, ie, inter, err, num_sms, st);
+    return walk_eps<D, MODE, false>(s, p, g, t, ie, inter, err, num_sms, st);
 }
 
 cudaError_t launch_walk(int dims, int precision, const State &s, const StepParams &p,
@@ -560,13 +594,13 @@ cudaError_t launch_walk(int dims, int precision, const State &s, const StepParam
         p.eps2 > 0.0f)
         return launch_warp_walk(dims, s, p, g, t, integrate_end, inter_count, err, num_sms, st);
     if (precision == GE_PREC_MIXED)
-        return dims == 2 ? walk_mode<2, GE_PREC_MIXED>(s, p, g, t, ie, inter_count, err, st)
-                         : walk_mode<3, GE_PREC_MIXED>(s, p, g, t, ie, inter_count, err, st);
+        return dims == 2 ? walk_mode<2, GE_PREC_MIXED>(s, p, g, t, ie, inter_count, err, num_sms, st)
+                         : walk_mode<3, GE_PREC_MIXED>(s, p, g, t, ie, inter_count, err, num_sms, st);
     if (dims == 2)
-        return exact ? walk_mode<2, GE_PREC_EXACT>(s, p, g, t, ie, inter_count, err, st)
-                     : walk_mode<2, GE_PREC_FAST>(s, p, g, t, ie, inter_count, err, st);
-    return exact ? walk_mode<3, GE_PREC_EXACT>(s, p, g, t, ie, inter_count, err, st)
-                 : walk_mode<3, GE_PREC_FAST>(s, p, g, t, ie, inter_count, err, st);
+        return exact ? walk_mode<2, GE_PREC_EXACT>(s, p, g, t, ie, inter_count, err, num_sms, st)
+                     : walk_mode<2, GE_PREC_FAST>(s, p, g, t, ie, inter_count, err, num_sms, st);
+    return exact ? walk_mode<3, GE_PREC_EXACT>(s, p, g, t, ie, inter_count, err, num_sms, st)
+                 : walk_mode<3, GE_PREC_FAST>(s, p, g, t, ie, inter_count, err, num_sms, st);
 }
 
 }  // namespace ge

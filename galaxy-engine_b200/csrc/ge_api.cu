@@ -134,7 +134,7 @@ struct ge_ctx {
     uint32_t *h_meta = nullptr;   // pinned copy of the tree meta words
     int64_t slots = 0;            // node slots of the last build (holes included)
     bool count_inter = false;
-    bool tree_ranges = false;   // the last build wrote the layout ranges (warp walk)
+    bool tree_warp = false;       // the last build wrote the warp walk's layout
     bool tree_valid = false;
     bool keys_valid = false;
     cudaEvent_t ev[8]{};
@@ -703,10 +703,11 @@ int enqueue_build(ge_ctx *c, bool fresh_keys = false) {
     StepParams p = step_params(c);
     // the optional layout arrays this build's readers need
     const bool temps = c->p.temp_enabled && c->b.temp;
+    const bool warp = warp_walk_on(p, c->p.precision, temps);
     p.layout_extras = (c->p.precision == GE_PREC_MIXED || temps ? kLayoutEntry : 0) |
-                      (c->p.walk_kind == 1 ? kLayoutRange : 0) |
-                      (c->p.dims == 3 && temps ? kLayoutPlain : 0);
-    c->tree_ranges = c->p.walk_kind == 1;
+                      (warp ? kLayoutRange : 0) |
+                      (c->p.dims == 3 && (temps || warp) ? kLayoutPlain : 0);
+    c->tree_warp = warp;
     const bool keyed = fresh_keys && c->p.leaf_cap >= 1 && c->p.leaf_cap <= (uint32_t)kKeyMaxCap;
     if (keyed)
         GE_CHECK(c, launch_key_build(c->p.dims, cur_state(c), p, c->g, c->b.ss.keys[0], c->b.tree,
@@ -738,8 +739,8 @@ int ensure_mode(ge_ctx *c) {
 
 int enqueue_walk(ge_ctx *c, bool integrate_end) {
     StepParams p = step_params(c);
-    // a tree built without the layout ranges takes the per-particle walk
-    if (!c->tree_ranges) p.walk_kind = 0;
+    // a tree built for the per-particle walk takes it
+    if (!c->tree_warp) p.walk_kind = 0;
     unsigned long long *cnt = nullptr;
     if (c->count_inter) {
         GE_CHECK(c, cudaMemsetAsync(c->b.d_inter, 0, sizeof(unsigned long long), c->stream));

@@ -227,7 +227,9 @@ constexpr int kLayoutEntry = 1, kLayoutRange = 2;
 // it: their steps hang on the chain through the temperature, not on the loads
 // that packed words save, and unpacking them lengthens it (walk, packed / plain,
 // us: 5k 315 / 293, 100k 554 / 522, 300k 1078 / 994, 700k 2343 / 2275; EXACT 300k
-// 1561 / 1464; without heat exchange 300k 445 / 637)
+// 1561 / 1464; without heat exchange 300k 445 / 637).  So does the 3D warp walk,
+// whose lanes go through short ranges on their own (30k 405 / 288, 300k 1105 /
+// 750, 1M 2684 / 1917).
 constexpr int kLayoutPlain = 4;
 constexpr int kMetaBigRoot = 14;   // tree meta word: some simulation's root size >= 1e19
 // tree meta word: a mass is negative or, in a periodic domain, something with
@@ -384,9 +386,13 @@ cudaError_t launch_direct(int dims, int precision, const State &s, const StepPar
                           const Segs &g, const uint2 *tiles, int64_t ntiles, bool integrate_end,
                           cudaStream_t st);
 // tree walk; integrate_end fuses integrateEnd (v += a*dt/2).  With
-// p.walk_kind == 1, GE_PREC_FAST with eps2 > 0 and without periodic wrap or
-// heat exchange runs the warp-cooperative walk (ge_wwalk.cu); everything else
-// the per-particle walk (ge_walk.cu)
+// p.walk_kind == 1, GE_PREC_FAST with eps2 > 0 (the warp walk stages a
+// particle's own term with its leaf, which adds zero only then) and without
+// periodic wrap or heat exchange runs the warp-cooperative walk (ge_wwalk.cu);
+// everything else the per-particle walk (ge_walk.cu)
+inline bool warp_walk_on(const StepParams &p, int precision, bool temps) {
+    return p.walk_kind == 1 && precision == GE_PREC_FAST && !p.periodic && !temps && p.eps2 > 0.0f;
+}
 cudaError_t launch_walk(int dims, int precision, const State &s, const StepParams &p,
                         const Segs &g, const Tree &t, bool integrate_end,
                         unsigned long long *inter_count, uint32_t *err, int num_sms,

@@ -588,10 +588,7 @@ cudaError_t launch_walk(int dims, int precision, const State &s, const StepParam
                         cudaStream_t st) {
     const int ie = integrate_end ? 1 : 0;
     const bool exact = precision == GE_PREC_EXACT;
-    // (the warp walk stages a particle's own term with its leaf, which adds
-    // zero only with eps2 > 0)
-    if (p.walk_kind == 1 && precision == GE_PREC_FAST && !p.periodic && !(s.temp && t.tv) &&
-        p.eps2 > 0.0f)
+    if (warp_walk_on(p, precision, s.temp && t.tv))
         return launch_warp_walk(dims, s, p, g, t, integrate_end, inter_count, err, num_sms, st);
     if (precision == GE_PREC_MIXED)
         return dims == 2 ? walk_mode<2, GE_PREC_MIXED>(s, p, g, t, ie, inter_count, err, num_sms, st)

@@ -103,14 +103,15 @@ __device__ __forceinline__ void eval_list(const WWSmem &sm, int nl, const float 
 }
 
 // One entry of the depth-first layout: its position/mass word, size^2 (nodes),
-// subtree successor, and whether it is a particle.
+// subtree successor, and whether it is a particle (3D builds write the plain
+// layout for this walk).
 template <int D>
 __device__ __forceinline__ void layout_entry(const Tree &t, uint32_t k, bool packed,
                                              uint32_t rs2_bits, float4 &A, float &s2,
                                              uint32_t &skip, bool &part) {
     A = __ldg(&t.src[k]);
-    if (packed) {
-        const uint32_t wb = D == 2 ? __float_as_uint(A.w) : __ldg(&((const uint32_t *)t.link)[k]);
+    if (D == 2 && packed) {
+        const uint32_t wb = __float_as_uint(A.w);
         part = packed_particle(wb);   // (massless nodes: mass 0, accepted below)
         s2 = packed_size2(wb, rs2_bits);
         skip = k + 1u + packed_ahead(wb);
@@ -190,7 +191,7 @@ k_warp_walk(State s, StepParams p, Segs g, Tree t, int integrate_end,
                                    : (uint32_t)((n - i0 + 31) / 32);
     const float eps2 = p.eps2, th2 = p.theta2;
     const float *pos[3] = {s.x, s.y, s.z};
-    const bool packed = __ldcg(&t.meta[kMetaWalkPacked]) != 0u;
+    const bool packed = D == 2 && __ldcg(&t.meta[kMetaWalkPacked]) != 0u;
     unsigned long long my_count = 0;
     while (true) {
         uint32_t c = kEmpty;   // the next chunk

@@ -18,36 +18,47 @@ namespace ge {
 
 constexpr int kPredThreads = 64;
 
-// the packed layout's word of entry k: 2D in the entry, 3D in the link array
-__device__ __forceinline__ uint32_t entry_word(const Tree &t, int D, uint32_t k) {
-    return D == 2 ? __float_as_uint(__ldg(&t.src[k]).w) : __ldg(&((const uint32_t *)t.link)[k]);
-}
-// size^2 of entry k (-1 for a particle); rs_bits: the simulation's root
-// size^2, for the packed layout
-__device__ __forceinline__ float entry_s2(const Tree &t, int D, uint32_t k, bool packed,
-                                          uint32_t rs_bits) {
-    if (!packed)
-        return D == 2 ? __ldg(&t.src[k]).w : __uint_as_float(__ldg(&((const uint2 *)t.link)[k]).y);
-    const uint32_t wb = entry_word(t, D, k);
-    if (packed_particle(wb)) return -1.0f;
-    if (packed_accepts(wb)) return -2.0f;   // a massless node
-    return packed_size2(wb, rs_bits);
-}
-// successor of entry k
-__device__ __forceinline__ uint32_t entry_skip(const Tree &t, int D, uint32_t k, bool packed) {
-    if (packed) return k + 1u + packed_ahead(entry_word(t, D, k));
-    return D == 2 ? __ldg(&((const uint32_t *)t.link)[k]) : __ldg(&((const uint2 *)t.link)[k]).x;
+// What the older walk asks of entry k: its successor, its size^2 and whether it
+// is a leaf (its first particle follows it).  PK: the packed layout's words (2D
+// in the entries, 3D in the link array), k's and the next entry's, asked for
+// together; rs_bits: the simulation's root size^2.
+template <int D, bool PK>
+__device__ __forceinline__ void entry(const Tree &t, uint32_t k, uint32_t last, uint32_t rs_bits,
+                                      const float4 &A, uint32_t &skip, float &s2, bool &leaf) {
+    const uint32_t k1 = min(k + 1u, last);
+    if constexpr (PK) {
+        const uint32_t w = D == 2 ? __float_as_uint(A.w) : __ldg(&((const uint32_t *)t.link)[k]);
+        const uint32_t w1 = D == 2 ? __float_as_uint(__ldg(&t.src[k1].w))
+                                   : __ldg(&((const uint32_t *)t.link)[k1]);
+        skip = k + 1u + packed_ahead(w);
+        s2 = packed_size2(w, rs_bits);   // a node with mass: its level is no marker
+        leaf = packed_particle(w1);
+    } else if constexpr (D == 2) {
+        const float s1 = __ldg(&t.src[k1].w);
+        skip = __ldg(&((const uint32_t *)t.link)[k]);
+        s2 = A.w;
+        leaf = s1 == -1.0f;
+    } else {
+        const uint2 l = __ldg(&((const uint2 *)t.link)[k]);
+        const float s1 = __uint_as_float(__ldg(&((const uint2 *)t.link)[k1].y));
+        skip = l.x;
+        s2 = __uint_as_float(l.y);
+        leaf = s1 == -1.0f;
+    }
+    leaf = leaf && k + 1u < skip;
 }
 
-template <int D>
+template <int D, bool PK>
 __device__ void old_force(const Tree &t, const StepParams &p, uint32_t begin, uint32_t end,
-                          float eps2, const float *pos, float pmass, float *F, bool packed,
-                          uint32_t rs_bits) {
+                          float eps2, const float *pos, float pmass, float *F, uint32_t rs_bits) {
     F[0] = F[1] = F[2] = 0.0f;
     uint32_t k = begin;
     while (k < end) {
         const float4 A = __ldg(&t.src[k]);
-        const uint32_t skip = entry_skip(t, D, k, packed);
+        uint32_t skip;
+        float s2;
+        bool leaf;   // a leaf's particles follow it in the layout
+        entry<D, PK>(t, k, end - 1u, rs_bits, A, skip, s2, leaf);
         const uint32_t nxt = max(k + 1, skip);   // always moves forward
         const float gm = D == 2 ? A.z : A.w;
         if (!(gm > 0.0f)) { k = nxt; continue; }   // gridMass <= 0: skip the subtree
@@ -64,9 +75,6 @@ __device__ void old_force(const Tree &t, const StepParams &p, uint32_t begin, ui
         float r2 = fadd(fmul(d[0], d[0]), fmul(d[1], d[1]));
         if (D == 3) r2 = fadd(r2, fmul(d[2], d[2]));
         r2 = fadd(r2, eps2);
-        // a leaf's particles follow it in the layout (size^2 = -1)
-        const bool leaf = k + 1 < skip && entry_s2(t, D, k + 1, packed, rs_bits) == -1.0f;
-        const float s2 = entry_s2(t, D, k, packed, rs_bits);
         if (s2 < fmul(p.theta2, r2) || leaf) {
             if (leaf && skip - k - 1 == 1u) {   // one particle: skip it when it sits on the probe
                 const float4 o = __ldg(&t.src[k + 1]);
@@ -88,22 +96,21 @@ __device__ void old_force(const Tree &t, const StepParams &p, uint32_t begin, ui
     }
 }
 
-template <int D>
-__global__ void __launch_bounds__(kPredThreads)
-k_predict(Tree t, StepParams p, const float4 *box, uint32_t begin, uint32_t end, float eps2,
-          int nprobes, const float *__restrict__ pos, const float *__restrict__ vel,
-          const float *__restrict__ mass, int steps, float *__restrict__ path) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= nprobes) return;
-    const bool packed = __ldg(&t.meta[kMetaWalkPacked]) != 0u;
-    const float rs = packed ? __ldg(box).w : 0.0f;   // the simulation's root size
+template <int D, bool PK>
+__device__ __forceinline__ void predict_one(const Tree &t, const StepParams &p, const float4 *box,
+                                            uint32_t begin, uint32_t end, float eps2, int q,
+                                            const float *__restrict__ pos,
+                                            const float *__restrict__ vel,
+                                            const float *__restrict__ mass, int steps,
+                                            float *__restrict__ path) {
+    const float rs = PK ? __ldg(box).w : 0.0f;   // the simulation's root size
     const uint32_t rs_bits = __float_as_uint(fmul(rs, rs));
     float ps[3] = {0.f, 0.f, 0.f}, v[3] = {0.f, 0.f, 0.f}, F[3];
 #pragma unroll
     for (int a = 0; a < D; a++) { ps[a] = pos[q * D + a]; v[a] = vel[q * D + a]; }
     const float m = mass[q], h = fmul(p.dt, 0.5f);
     for (int s = 0; s < steps; s++) {
-        old_force<D>(t, p, begin, end, eps2, ps, m, F, packed, rs_bits);
+        old_force<D, PK>(t, p, begin, end, eps2, ps, m, F, rs_bits);
 #pragma unroll
         for (int a = 0; a < D; a++) v[a] = fadd(v[a], fmul(fdiv(F[a], m), h));
 #pragma unroll
@@ -118,12 +125,26 @@ k_predict(Tree t, StepParams p, const float4 *box, uint32_t begin, uint32_t end,
                 else if (ps[a] >= hi) ps[a] = fsub(ps[a], p.domain[a]);
             }
         }
-        old_force<D>(t, p, begin, end, eps2, ps, m, F, packed, rs_bits);
+        old_force<D, PK>(t, p, begin, end, eps2, ps, m, F, rs_bits);
 #pragma unroll
         for (int a = 0; a < D; a++) v[a] = fadd(v[a], fmul(fdiv(F[a], m), h));
 #pragma unroll
         for (int a = 0; a < D; a++) path[((size_t)q * steps + s) * D + a] = ps[a];
     }
+}
+
+// the loop once per layout, chosen here rather than at every entry
+template <int D>
+__global__ void __launch_bounds__(kPredThreads)
+k_predict(Tree t, StepParams p, const float4 *box, uint32_t begin, uint32_t end, float eps2,
+          int nprobes, const float *__restrict__ pos, const float *__restrict__ vel,
+          const float *__restrict__ mass, int steps, float *__restrict__ path) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= nprobes) return;
+    if (__ldg(&t.meta[kMetaWalkPacked]) != 0u)
+        predict_one<D, true>(t, p, box, begin, end, eps2, q, pos, vel, mass, steps, path);
+    else
+        predict_one<D, false>(t, p, box, begin, end, eps2, q, pos, vel, mass, steps, path);
 }
 
 cudaError_t launch_predict(int dims, const Tree &t, const StepParams &p, const float4 *box,

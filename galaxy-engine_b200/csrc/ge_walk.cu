@@ -43,6 +43,12 @@ namespace ge {
 // link had 8 bytes, 1M 1.65 ms against 1.78; with packed links 256 takes 1.56,
 // 250k 483 us against 537, 60k 188 against 275, 16k 142 against 227.)
 constexpr int kWalkThreads = 256, kWalkThreads2D = 512, kWalkThreadsRows = 1024;
+// Whether a build packs its 3D entries (k_build decides): a tree of this many
+// particles, with some 0.7 nodes for each, within the words' successors.
+// Where the guess is wrong the walk is a slower one with the same bits.
+static bool walk_packs(const StepParams &p) {
+    return p.min_size >= 1e-18f && p.n < (int)((1u << kPackSkipBits) / 17 * 10);
+}
 // 3D EXACT, MIXED and heat exchange: blocks of 1024 share more still, and take
 // less time where their last row (one block on every SM) is at least nine tenths
 // full; with a row that is not, the SMs with one block more than others cost more
@@ -53,10 +59,18 @@ constexpr int kWalkThreads = 256, kWalkThreads2D = 512, kWalkThreadsRows = 1024;
 // threads (faster below its six blocks per SM: 50k 672 / 1057) and 32 with 1024,
 // where a row alone on the SMs is slow, so two rows have to be full: 285k 3205 /
 // 2365, 300k 3141 / 2483, 450k 3707 / 4164, 605k 5161 / 4670, 900k 7356 / 6928.
-static bool walk_rows_full(int mode, int n, int num_sms) {
+// FAST in the plain layout, whose links have 8 bytes, from two rows on whether
+// full or not: theta 0.5 450k 3282 / 2708, 1M 6208 / 4860, 0.7 1M 1763 / 1645, 1.0
+// 1M 565 / 590 (by pairs 3156, 5242, 1823, 700).
+static bool walk_rows(const StepParams &p, int mode, bool temp, int num_sms) {
+    const int blocks = (p.n - p.i0 + kWalkThreadsRows - 1) / kWalkThreadsRows;
+    if (blocks < 1) return false;
+    if (mode == GE_PREC_FAST && !temp) {
+        if (walk_packs(p)) return false;
+        if (blocks > 2 * num_sms) return true;
+    }
     const int row = mode == GE_PREC_MIXED ? 2 * num_sms : num_sms;
-    const int last = ((n + kWalkThreadsRows - 1) / kWalkThreadsRows - 1) % row + 1;
-    return n > 0 && 10 * last >= 9 * row;
+    return 10 * ((blocks - 1) % row + 1) >= 9 * row;
 }
 // 2D, by the launch's particles.  While SMs are left over, larger blocks share
 // more (256 -> 512 threads, us: 2k 38.9 -> 36.8, 6k 49.2 -> 45.1, 12k 53.3 ->
@@ -384,13 +398,17 @@ k_walk(State s, StepParams p, Segs g, Tree t, int integrate_end, unsigned long l
 // the same bits.  Half the threads and a longer step, so it pays where the walks
 // are long and many: walk (us), single / pairs, theta 0.7: 60k 190 / 227, 150k
 // 268 / 283, 200k 383 / 332, 250k 479 / 397, 1M 1558 / 1334; theta 0.5 1M 5172 /
-// 3588; theta 1.0 150k 119 / 150, 400k 283 / 275; periodic (a warp that holds
-// both kinds of particles runs both loops) 250k 477 / 520, 1M 1580 / 1438.  In
-// 2D, bound by instructions as much as by L1, it does not (1M 277 / 285).
+// 3588; theta 1.0 150k 119 / 150, 400k 283 / 275.  Many small systems in one
+// launch gain as one large one does (theta 0.8, 400 of up to 2k 335 / 314, 100 of
+// up to 15k 516 / 469).  Periodic systems gain where few of their offsets wrap
+// (domain twice the system 250k 495 / 407, 1M 1572 / 1381) and lose where most do
+// (a full domain 250k 342 / 372, 1M 1158 / 1228).  Plain entries gain at no size
+// worth it (walk_rows), nor does 2D, bound by instructions as much as by L1 (1M
+// 277 / 285).
 constexpr int kPairThreads = 128;
 static bool walk_pairs(const StepParams &p) {
     const int n = p.n - p.i0;
-    return n >= 400000 || (n >= 200000 && p.theta <= 0.8f && !p.periodic);
+    return walk_packs(p) && (n >= 400000 || (n >= 200000 && p.theta <= 0.8f && !p.periodic));
 }
 
 // entry k in either layout: whether a particle at squared distance r2
@@ -550,9 +568,8 @@ static cudaError_t walk_one(const State &s, const StepParams &p, const Segs &g, 
         return go(std::integral_constant<int, kWalkThreads2D>{},
                   MODE != GE_PREC_MIXED ? walk_threads_2d(n) : kWalkThreads);
     } else {
-        if constexpr (MODE != GE_PREC_FAST || TEMP)
-            if (walk_rows_full(MODE, n, num_sms))
-                return go(std::integral_constant<int, kWalkThreadsRows>{}, kWalkThreadsRows);
+        if (walk_rows(p, MODE, TEMP, num_sms))
+            return go(std::integral_constant<int, kWalkThreadsRows>{}, kWalkThreadsRows);
         return go(std::integral_constant<int, kWalkThreads>{}, kWalkThreads);
     }
 }

@@ -1,7 +1,9 @@
 """GPU: the 3D walk's block sizes.
 
-EXACT, MIXED (per particle) and heat-exchange walks take blocks of 1024 threads
-where these fill the SMs evenly, of 256 elsewhere.  A particle's walk does not
+EXACT, MIXED (per particle) and heat-exchange walks, and FAST ones over plain
+entries (here from a minimum size too small for packed ones), take blocks of 1024
+threads where these fill the SMs evenly, the last also from two rows on, and of
+256 elsewhere.  A particle's walk does not
 depend on it: simulations on both sides of the rule's limits, alone, equal the
 same simulation in a batch, whose launch takes another size, bit for bit.
 """
@@ -18,7 +20,9 @@ ROW = 148 * 1024   # a full row of blocks
 @pytest.mark.parametrize("mode,n", [("EXACT", 133 * 1024), ("EXACT", 133 * 1024 + 1), ("EXACT", ROW),
                                     ("EXACT", ROW + 1), ("heat", 134 * 1024), ("heat", ROW),
                                     ("EXACT heat", ROW - 3), ("EXACT periodic", ROW),
-                                    ("MIXED", 266 * 1024), ("MIXED", 266 * 1024 + 1)])
+                                    ("MIXED", 266 * 1024), ("MIXED", 266 * 1024 + 1),
+                                    ("plain", ROW), ("plain", 2 * ROW), ("plain", 2 * ROW + 1),
+                                    ("plain", 3 * ROW // 2)])
 def test_alone_equals_batch(ge, ics, mode, n):
     kw = dict(G=1.0, theta=1.0, eps2=0.01, dt=1e-3)
     if "EXACT" in mode:
@@ -27,6 +31,8 @@ def test_alone_equals_batch(ge, ics, mode, n):
         kw.update(precision=ge.PREC_MIXED, group_size=0, leaf_cap=4)
     if "heat" in mode:
         kw.update(temp_enabled=1)
+    if mode == "plain":
+        kw.update(min_size=1e-20)
     if "periodic" in mode:
         kw.update(periodic=1, domain=(60.0,) * 3)
     st, other = ics.plummer3d(n, seed=3), ics.plummer3d(5000, seed=4)

@@ -749,7 +749,7 @@ int enqueue_walk(ge_ctx *c, bool integrate_end) {
     if (group_walk_on(c)) {
         GE_CHECK(c, launch_group_walk(c->p.dims, cur_state(c), p, c->g, mixed_view(c),
                                       integrate_end, cnt, c->b.tree.meta + 10, c->d_err,
-                                      c->stream));
+                                      c->num_sms, c->stream));
         return GE_OK;
     }
     State s = cur_state(c);
@@ -2040,7 +2040,7 @@ int ge_energy_f64(ge_ctx *c, double *out) {
     GE_CHECK(c, cudaMallocAsync((void **)&d, sizeof(double) * 6, c->stream));
     StepParams p = step_params(c);
     GE_CHECK(c, launch_group_potential(c->p.dims, cur_state(c), p, c->g, mixed_view(c),
-                                       c->b.tree.meta + 10, c->d_err, d, c->stream));
+                                       c->b.tree.meta + 10, c->d_err, d, c->num_sms, c->stream));
     GE_CHECK(c, launch_sums_f64(c->p.dims, cur_state(c), (int)c->n, d + 1, c->stream));
     double h[6];
     GE_CHECK(c, cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, c->stream));

@@ -32,6 +32,7 @@
 // traversal order, so the interaction set is deterministic; only the FP32
 // summation order within a list pass follows the traversal.
 #include <cfloat>
+#include <type_traits>
 
 #include "ge_bh.h"
 #include "ge_device.cuh"
@@ -548,12 +549,22 @@ __global__ void k_make_groups(Tree t, uint32_t GS) {
     }
 }
 
+// One particle per lane: how the walk hides its latency.  Small launches load
+// the next candidates ahead, in the registers of four blocks per SM; from some
+// 200,000 particles on six blocks per SM hide more, which have no registers for
+// that and stage a round's nodes before its children are pushed (BUSY).  Walk of
+// groups of 32 (us, ahead / BUSY): 3D theta 0.7 10k 172 / 199, 100k 500 / 524, 200k
+// 868 / 829, 500k 1966 / 1772, 1M 3855 / 3446, 2D 60k 61 / 69, 200k 139 / 137, 1M 574 /
+// 549.
+constexpr int kBusyGroups = 200000;
+static bool gw_busy(int n) { return n >= kBusyGroups; }
+
 // GSC: the group size in 32-particle chunks.  A work item is PPL = min(GSC, 2)
 // of a group's chunks: every item of a group takes the whole group's box, so
 // it meets the same sources in the same order as one warp that walked for all
 // of them would, and an item without particles is passed over.
-template <int D, int GSC, bool COUNT, bool POT = false>
-__global__ void __launch_bounds__(kGWThreads, 4)
+template <int D, int GSC, bool COUNT, bool POT = false, bool BUSY = false>
+__global__ void __launch_bounds__(kGWThreads, BUSY ? 6 : 4)
 k_group_walk(State s, StepParams p, Segs sg_tab, Tree t, int integrate_end,
              unsigned long long *inter, uint32_t *err, double *epot = nullptr) {
     dep_wait();
@@ -628,8 +639,8 @@ k_group_walk(State s, StepParams p, Segs sg_tab, Tree t, int integrate_end,
 #pragma unroll
             for (int a = 0; a < D; a++) g.x[k][a] -= oc[a];
         int nl = 0, pl = 0;
-        // a round's candidates, one per lane, and what their test needs; the
-        // next round's are loaded before this round's lists are filled and
+        // a round's candidates, one per lane, and what their test needs; unless
+        // BUSY the next round's are loaded before this round's lists are filled and
         // evaluated, so their latency passes meanwhile
         uint32_t top = 0, c = lane == 0 ? sg : kEmpty;   // the simulation's root node slot
         bool spilled = false;   // warp-uniform: the stack is in wl (global)
@@ -660,47 +671,65 @@ k_group_walk(State s, StepParams p, Segs sg_tab, Tree t, int integrate_end,
                     kind = b2 < dm ? 1 : (inf.y ? 3 : 2);
                 }
             }
-            // 1. children of opened internal nodes onto the work stack
-            const uint32_t nch = kind == 3 ? (uint32_t)__popc(inf.y) : 0u;
-            uint32_t incl = nch;
+            // children of opened internal nodes onto the work stack (false: it is
+            // full), from whose top the next round's candidates come
+            auto push = [&]() {
+                const uint32_t nch = kind == 3 ? (uint32_t)__popc(inf.y) : 0u;
+                uint32_t incl = nch;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= (unsigned)o) incl += v;
-            }
-            const uint32_t tot = __shfl_sync(0xffffffffu, incl, 31);
-            if (!spilled && top + tot > GWShared<D>::value) {   // warp-uniform: move to wl
-                for (uint32_t q = lane; q < top; q += 32) wl[q] = stk[q];
-                spilled = true;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= (unsigned)o) incl += v;
+                }
+                const uint32_t tot = __shfl_sync(0xffffffffu, incl, 31);
+                if (!spilled && top + tot > GWShared<D>::value) {   // warp-uniform: move to wl
+                    for (uint32_t q = lane; q < top; q += 32) wl[q] = stk[q];
+                    spilled = true;
+                    __syncwarp();
+                }
+                if (top + tot > kGWStack) return false;   // warp-uniform
+                if (spilled)
+                    for (uint32_t q = 0; q < nch; q++) wl[top + incl - nch + q] = inf.x + q;
+                else
+                    for (uint32_t q = 0; q < nch; q++) stk[top + incl - nch + q] = inf.x + q;
+                top += tot;
                 __syncwarp();
-            }
-            if (top + tot > kGWStack) {   // warp-uniform
-                overflow = true;
-                break;
-            }
-            if (spilled)
-                for (uint32_t q = 0; q < nch; q++) wl[top + incl - nch + q] = inf.x + q;
-            else
-                for (uint32_t q = 0; q < nch; q++) stk[top + incl - nch + q] = inf.x + q;
-            top += tot;
-            __syncwarp();
-            // an accepted node's moments, then the next round's candidates
+                return true;
+            };
+            auto take = [&]() {
+                const uint32_t some = min(top, 32u);
+                top -= some;
+                c = lane < some ? (spilled ? __ldcg(&wl[top + lane]) : stk[top + lane]) : kEmpty;
+            };
+            // an accepted node's entry and moments
             const uint32_t ce = c;
             const float4 Ae = A;
             float4 Bq = make_float4(0.f, 0.f, 0.f, 0.f), Cq = Bq;
             float Eq = 0.0f;
-            if (kind == 1) {
+            auto moments = [&]() {
+                if (kind != 1) return;
                 Bq = __ldg(&t.gq0[ce]);
                 if (D == 3) Cq = __ldg(&t.gq1[ce]);
                 Eq = D == 3 ? E2.x : __ldg(&t.gq2[ce]).x;
+            };
+            uint32_t pc = 0, pbeg = 0;   // the particles of an opened leaf
+            auto leaf = [&]() {
+                pc = kind == 2 ? inf.w - inf.z : 0u;
+                pbeg = inf.z;
+            };
+            if (!BUSY) {
+                if (!push()) {
+                    overflow = true;
+                    break;
+                }
+                moments();
+                leaf();
+                take();
+                load();
+            } else {
+                moments();
             }
-            // particles of opened leaves
-            const uint32_t pc = kind == 2 ? inf.w - inf.z : 0u, pbeg = inf.z;
-            const uint32_t take = min(top, 32u);
-            top -= take;
-            c = lane < take ? (spilled ? __ldcg(&wl[top + lane]) : stk[top + lane]) : kEmpty;
-            load();
-            // 2. accepted nodes into the node list
+            // accepted nodes into the node list
             const unsigned accb = __ballot_sync(0xffffffffu, kind == 1);
             if (nl + __popc(accb) > kGWNodes) {
                 eval_nodes<D, PPL, DUP, COUNT, POT>(sm, nl, g, eps2, nk);
@@ -728,7 +757,15 @@ k_group_walk(State s, StepParams p, Segs sg_tab, Tree t, int integrate_end,
                 put_node<D, DUP>(sm, q, v);
             }
             nl += __popc(accb);
-            // 3. particles of opened leaves into the particle list, which is
+            if (BUSY) {
+                if (!push()) {
+                    overflow = true;
+                    break;
+                }
+                take();
+                leaf();
+            }
+            // particles of opened leaves into the particle list, which is
             // evaluated whenever it is full: the leaves' particles are numbered
             // through (in lane order) and each lane takes every 32nd of them
             if (__any_sync(0xffffffffu, pc > 0u)) {
@@ -766,6 +803,7 @@ k_group_walk(State s, StepParams p, Segs sg_tab, Tree t, int integrate_end,
                 }
             }
             __syncwarp();
+            if (BUSY) load();
         }
         if (overflow) {
             if (lane == 0) set_err(err, kErrStack);
@@ -822,11 +860,11 @@ static int grid_blocks(int n) {
     return b < 1 ? 1 : b;
 }
 
-template <int D, int GSC, bool COUNT>
+template <int D, int GSC, bool COUNT, bool POT = false, bool BUSY = false>
 static int resident_blocks() {
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_group_walk<D, GSC, COUNT>,
-                                                      kGWThreads, 0) != cudaSuccess)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+            &per_sm, k_group_walk<D, GSC, COUNT, POT, BUSY>, kGWThreads, 0) != cudaSuccess)
         return 0;
     return per_sm;
 }
@@ -839,6 +877,8 @@ static int most_resident() {
     m = max(m, resident_blocks<D, 1, true>());
     m = max(m, resident_blocks<D, 2, true>());
     m = max(m, resident_blocks<D, 4, true>());
+    m = max(m, resident_blocks<D, 1, false, false, true>());
+    m = max(m, resident_blocks<D, 1, true, false, true>());
     return m;
 }
 
@@ -850,69 +890,88 @@ int group_walk_warps(int dims, int num_sms) {
 
 uint32_t group_walk_stack_entries() { return kGWStack; }
 
+// Blocks of a walk: those it keeps resident, at most one per four groups, which
+// number at most n; the work stacks, one per warp, bound them too.
+template <int D, int GSC, bool COUNT, bool POT, bool BUSY>
+static int gw_blocks(const Tree &t, int n, int num_sms) {
+    static const int per_sm = resident_blocks<D, GSC, COUNT, POT, BUSY>();
+    const int64_t stacks = t.wl_warps / kGWWarps, groups = ((int64_t)n + kGWWarps - 1) / kGWWarps;
+    const int64_t resident = per_sm > 0 ? (int64_t)per_sm * num_sms : stacks;
+    return (int)max((int64_t)1, min(min(stacks, resident), groups));
+}
+
+template <int D, int GSC, bool COUNT, bool BUSY>
+static cudaError_t gw_walk(const State &s, const StepParams &p, const Segs &g, const Tree &t, int ie,
+                           unsigned long long *inter, uint32_t *err, int num_sms, cudaStream_t st) {
+    double *no_pot = nullptr;
+    return launch_dep(k_group_walk<D, GSC, COUNT, false, BUSY>,
+                      gw_blocks<D, GSC, COUNT, false, BUSY>(t, p.n, num_sms), kGWThreads, st, s, p,
+                      g, t, ie, inter, err, no_pot);
+}
+
 template <int D, int GSC, bool COUNT>
 static cudaError_t gw_launch(const State &s, const StepParams &p, const Segs &g, const Tree &t,
-                             int ie, unsigned long long *inter, uint32_t *err, cudaStream_t st) {
+                             int ie, unsigned long long *inter, uint32_t *err, int num_sms,
+                             cudaStream_t st) {
     cudaError_t e = launch_dep(k_make_groups<D>, grid_blocks(p.n), 256, st, t, 32u * GSC);
     if (e != cudaSuccess) return e;
-    // one work stack per warp bounds the grid; groups number at most n
-    int blocks = (int)(t.wl_warps / kGWWarps);
-    const int64_t want = ((int64_t)p.n + kGWWarps - 1) / kGWWarps;
-    if (blocks > want) blocks = (int)want;
-    if (blocks < 1) blocks = 1;
-    double *no_pot = nullptr;
-    return launch_dep(k_group_walk<D, GSC, COUNT>, blocks, kGWThreads, st, s, p, g, t, ie, inter, err,
-                      no_pot);
+    if constexpr (GSC == 1)
+        if (gw_busy(p.n)) return gw_walk<D, GSC, COUNT, true>(s, p, g, t, ie, inter, err, num_sms, st);
+    return gw_walk<D, GSC, COUNT, false>(s, p, g, t, ie, inter, err, num_sms, st);
 }
 
 template <int D>
 static cudaError_t gw_dims(const State &s, const StepParams &p, const Segs &g, const Tree &t,
-                           int ie, unsigned long long *inter, uint32_t *err, cudaStream_t st) {
+                           int ie, unsigned long long *inter, uint32_t *err, int num_sms,
+                           cudaStream_t st) {
     if (inter) {
-        if (p.group_size >= 128) return gw_launch<D, 4, true>(s, p, g, t, ie, inter, err, st);
-        if (p.group_size >= 64) return gw_launch<D, 2, true>(s, p, g, t, ie, inter, err, st);
-        return gw_launch<D, 1, true>(s, p, g, t, ie, inter, err, st);
+        if (p.group_size >= 128) return gw_launch<D, 4, true>(s, p, g, t, ie, inter, err, num_sms, st);
+        if (p.group_size >= 64) return gw_launch<D, 2, true>(s, p, g, t, ie, inter, err, num_sms, st);
+        return gw_launch<D, 1, true>(s, p, g, t, ie, inter, err, num_sms, st);
     }
-    if (p.group_size >= 128) return gw_launch<D, 4, false>(s, p, g, t, ie, inter, err, st);
-    if (p.group_size >= 64) return gw_launch<D, 2, false>(s, p, g, t, ie, inter, err, st);
-    return gw_launch<D, 1, false>(s, p, g, t, ie, inter, err, st);
+    if (p.group_size >= 128) return gw_launch<D, 4, false>(s, p, g, t, ie, inter, err, num_sms, st);
+    if (p.group_size >= 64) return gw_launch<D, 2, false>(s, p, g, t, ie, inter, err, num_sms, st);
+    return gw_launch<D, 1, false>(s, p, g, t, ie, inter, err, num_sms, st);
 }
 
 template <int D, int PPL>
 static cudaError_t gw_pot(const State &s, const StepParams &p, const Segs &g, const Tree &t,
-                          uint32_t *err, double *epot, cudaStream_t st) {
+                          uint32_t *err, double *epot, int num_sms, cudaStream_t st) {
     k_make_groups<D><<<grid_blocks(p.n), 256, 0, st>>>(t, 32u * PPL);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    int blocks = (int)(t.wl_warps / kGWWarps);
-    const int64_t want = ((int64_t)p.n + kGWWarps - 1) / kGWWarps;
-    if (blocks > want) blocks = (int)want;
-    if (blocks < 1) blocks = 1;
-    k_group_walk<D, PPL, false, true><<<blocks, kGWThreads, 0, st>>>(s, p, g, t, 0, nullptr, err,
-                                                                     epot);
+    auto go = [&](auto busy) {
+        constexpr bool BUSY = decltype(busy)::value;
+        k_group_walk<D, PPL, false, true, BUSY>
+            <<<gw_blocks<D, PPL, false, true, BUSY>(t, p.n, num_sms), kGWThreads, 0, st>>>(
+                s, p, g, t, 0, nullptr, err, epot);
+    };
+    if (gw_busy(p.n)) go(std::true_type{});
+    else go(std::false_type{});
     return cudaGetLastError();
 }
 
 cudaError_t launch_group_potential(int dims, const State &s, const StepParams &p, const Segs &g,
                                    const Tree &t, uint32_t *counter, uint32_t *err, double *epot,
-                                   cudaStream_t st) {
+                                   int num_sms, cudaStream_t st) {
     if (!t.wl || !t.grp || t.wl_warps < (uint32_t)kGWWarps) return cudaErrorInvalidValue;
     cudaError_t e = cudaMemsetAsync(counter, 0, 2 * sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(epot, 0, sizeof(double), st)) != cudaSuccess) return e;
-    return dims == 2 ? gw_pot<2, 1>(s, p, g, t, err, epot, st) : gw_pot<3, 1>(s, p, g, t, err, epot, st);
+    return dims == 2 ? gw_pot<2, 1>(s, p, g, t, err, epot, num_sms, st)
+                     : gw_pot<3, 1>(s, p, g, t, err, epot, num_sms, st);
 }
 
 cudaError_t launch_group_walk(int dims, const State &s, const StepParams &p, const Segs &g,
                               const Tree &t, bool integrate_end, unsigned long long *inter_count,
-                              uint32_t *counter, uint32_t *err, cudaStream_t st) {
+                              uint32_t *counter, uint32_t *err, int num_sms, cudaStream_t st) {
     if (!t.wl || !t.grp || t.wl_warps < (uint32_t)kGWWarps) return cudaErrorInvalidValue;
     // counter[0]: next group to walk, counter[1]: groups made
     cudaError_t e = cudaMemsetAsync(counter, 0, 2 * sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
     const int ie = integrate_end ? 1 : 0;
-    return dims == 2 ? gw_dims<2>(s, p, g, t, ie, inter_count, err, st)
-                     : gw_dims<3>(s, p, g, t, ie, inter_count, err, st);
+    return dims == 2 ? gw_dims<2>(s, p, g, t, ie, inter_count, err, num_sms, st)
+                     : gw_dims<3>(s, p, g, t, ie, inter_count, err, num_sms, st);
 }
 
 }  // namespace ge

@@ -374,11 +374,11 @@ int group_walk_warps(int dims, int num_sms);
 // is written
 cudaError_t launch_group_potential(int dims, const State &s, const StepParams &p, const Segs &g,
                                    const Tree &t, uint32_t *counter, uint32_t *err, double *epot,
-                                   cudaStream_t st);
+                                   int num_sms, cudaStream_t st);
 uint32_t group_walk_stack_entries();
 cudaError_t launch_group_walk(int dims, const State &s, const StepParams &p, const Segs &g,
                               const Tree &t, bool integrate_end, unsigned long long *inter_count,
-                              uint32_t *counter, uint32_t *err, cudaStream_t st);
+                              uint32_t *counter, uint32_t *err, int num_sms, cudaStream_t st);
 // O(N^2) direct sum of the segments listed by tiles[ntiles] ({segment,
 // first particle}, kDirectTile particles each, inside one segment), fused
 // with integrateEnd like the walk

@@ -75,14 +75,17 @@ static bool walk_rows(const StepParams &p, int mode, bool temp, int num_sms) {
 // 2D, by the launch's particles.  While SMs are left over, larger blocks share
 // more (256 -> 512 threads, us: 2k 38.9 -> 36.8, 6k 49.2 -> 45.1, 12k 53.3 ->
 // 49.2, 20k 55.3 -> 53.8, 28k 55.8 -> 54.3, 36k the same; with heat exchange 12k
-// 133 -> 126).  Between one and four blocks of 256 per SM some SMs have one more
-// than others, which smaller blocks even out (256 -> 128: 45k 57.3 -> 55.3, 65k
-// 57.3 -> 53.2, 90k 57.5 -> 55.3, 130k 56.7 -> 55.3; with heat exchange 65k 139 ->
-// 131; 36k the same, 190k 65.5 -> 66.6).  3D gains on neither side (20k 157.7,
-// 159.7 with 512; 65k 178.2, 181.7 with 128).
-static int walk_threads_2d(int n) {
-    constexpr int kSms = 148;
-    return n <= 64 * 512 ? 512 : n > kSms * 256 && n <= 4 * kSms * 256 ? 128 : 256;
+// 133 -> 126; 10 disks of up to 4k 43.1 -> 41.0).  Between one and four blocks of
+// 256 per SM some SMs have one more than others, which smaller blocks even out for
+// one simulation (256 -> 128: 45k 57.3 -> 55.3, 65k 57.3 -> 53.2, 90k 57.5 -> 55.3,
+// 130k 56.7 -> 55.3; theta 0.5 65k 91.0 -> 85.5, 1.0 100k 36.4 -> 37.4; with heat
+// exchange 65k 139 -> 131; 36k the same, 190k 65.5 -> 66.6).  In a batch their
+// walks share more than that (128 -> 256: 64 disks of up to 1.5k 44.0 -> 41.6, 18 of
+// up to 16k 52.1 -> 48.1, 14 of up to 32k 54.8 -> 51.7).  3D gains on neither side
+// (20k 157.7, 159.7 with 512; 65k 178.2, 181.7 with 128).
+static int walk_threads_2d(int n, bool alone, int num_sms) {
+    if (n <= 64 * 512) return 512;
+    return alone && n > num_sms * 256 && n <= 4 * num_sms * 256 ? 128 : 256;
 }
 
 __device__ __forceinline__ float wrap_d(float d, float dom, float hd) {
@@ -566,7 +569,7 @@ static cudaError_t walk_one(const State &s, const StepParams &p, const Segs &g, 
     };
     if constexpr (D == 2) {
         return go(std::integral_constant<int, kWalkThreads2D>{},
-                  MODE != GE_PREC_MIXED ? walk_threads_2d(n) : kWalkThreads);
+                  MODE != GE_PREC_MIXED ? walk_threads_2d(n, g.S == 1, num_sms) : kWalkThreads);
     } else {
         if (walk_rows(p, MODE, TEMP, num_sms))
             return go(std::integral_constant<int, kWalkThreadsRows>{}, kWalkThreadsRows);

@@ -948,10 +948,9 @@ __device__ bool build_small_subtree_smem(const State &s, const StepParams &p, Tr
 // Whether a node's centre of mass, or a particle of a leaf, lies outside its
 // simulation's root box by more than kBoxSlack of half the domain: the periodic
 // walk leaves the wrap out only while nothing does (a leaf's plain sums drift
-// with its particles).  A function of its own, or its registers would cost the
-// scatter of systems that are not periodic (build of 16k 85.2 -> 86.8 us).
+// with its particles).
 template <int D>
-__device__ __noinline__ bool outside_box(const float *x, const float *y, const float *z, float4 box,
+__device__ __forceinline__ bool outside_box(const float *x, const float *y, const float *z, float4 box,
                                          float3 half, uint4 inf, float4 w, bool massless) {
     auto beyond = [&](float px, float py, float pz) {
         const float v[3] = {px, py, pz}, lo[3] = {box.x, box.y, box.z}, h[3] = {half.x, half.y, half.z};
@@ -1001,10 +1000,6 @@ __device__ __forceinline__ void scatter_entry(const State &s, const StepParams &
     const float nm = D == 2 ? w.z : w.w;
     const bool massless = nm <= 0.0f;
     bool negative = nm < 0.0f;   // its centres may lie anywhere
-    if (p.periodic &&
-        outside_box<D>(s.x, s.y, s.z, g.box[g.seg_of ? g.seg_of[inf.z] : 0u],
-                       make_float3(p.half_domain[0], p.half_domain[1], p.half_domain[2]), inf, w, massless))
-        t.meta[kMetaMayWrap] = 1u;
     if (massless) {
         // gridMass <= 0: the reference skips the whole subtree.  As a source
         // it is accepted by every test (size^2 = -2; particles have -1),
@@ -1570,6 +1565,18 @@ k_build(State s, StepParams p, Segs g, Tree t, uint32_t *err, int keyed) {
                              packed);
         }
     }
+    // (a pass of its own: inside the scatter its registers cost the systems that
+    // are not periodic 1 to 2 us)
+    if (p.periodic)
+        for (uint32_t k = gtid; k < slots; k += nthreads) {
+            const uint4 inf = __ldcg(&t.info[k]);
+            if (inf.w == 0u) continue;
+            const float4 w = __ldcg(&t.walk[k]);
+            if (outside_box<D>(s.x, s.y, s.z, g.box[g.seg_of ? g.seg_of[inf.z] : 0u],
+                               make_float3(p.half_domain[0], p.half_domain[1], p.half_domain[2]), inf, w,
+                               (D == 2 ? w.z : w.w) <= 0.0f))
+                t.meta[kMetaMayWrap] = 1u;
+        }
     // the last block to finish stamps the end of the build
     __syncthreads();
     if (threadIdx.x == 0) {

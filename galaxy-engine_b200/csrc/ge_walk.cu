@@ -139,8 +139,9 @@ template <> struct LinkOf<3> { using T = uint2; };
 // exactly zero.  x and y go through packed operations (f32x2), each rounded as
 // the scalar one.  The loads' L1 wavefronts bound it (79 % of peak; 6.7 per
 // load, the lanes of a warp at some five entries), so a quarter fewer
-// instructions give little: 1M at theta 0.7 278 -> 276 us, 283 in the general
-// loop.
+// instructions give little, and nothing below 100k particles: against the
+// general loop 1M at theta 0.5 507 -> 503 us, 0.7 290 -> 282, 1.0 165 -> 159, 2M at
+// 0.7 546 -> 527.
 __device__ __forceinline__ void walk_packed2(const float4 *__restrict__ src, uint32_t k,
                                              uint32_t end, uint32_t rs2_bits, const float *pi,
                                              float eps2, float th2, float *f) {

@@ -245,7 +245,8 @@ k_walk(State s, StepParams p, Segs g, Tree t, int integrate_end, unsigned long l
                 // includes 1 / theta
                 bool acc;
                 if constexpr (PK) acc = always || s2 < fmul(th2, r2);   // as -1 / -2 would
-                else acc = MODE == GE_PREC_MIXED ? s2 < r2 : s2 < fmul(th2, r2);
+                else if constexpr (MODE == GE_PREC_MIXED) acc = s2 < r2;
+                else acc = s2 < 0.0f || s2 < fmul(th2, r2);   // (a particle whose r2 is no number, too)
                 if (kSelfTest) {
                     // heat exchange (physics.cpp:145-158, 183-191): an accepted node
                     // with mass, or any other particle of an opened leaf (massless
@@ -426,7 +427,8 @@ __device__ __forceinline__ bool entry_accepts3(const Tree &t, uint32_t k, bool p
     }
     const uint2 l = __ldg(&((const uint2 *)t.link)[k]);
     nxt = max(k + 1u, l.x);   // a particle's successor is k + 1
-    return __uint_as_float(l.y) < th2r2;
+    const float s2 = __uint_as_float(l.y);
+    return s2 < 0.0f || s2 < th2r2;
 }
 
 template <bool PER>
